@@ -52,6 +52,8 @@ CUDA_SOURCES = [
     "ss_voxel.cu",
     "ss_push.cu",
     "ss_push_plan.cpp",
+    "ss_tile.cu",
+    "ss_tile_plan.cpp",
     "ss_capi.cu",
 ]
 

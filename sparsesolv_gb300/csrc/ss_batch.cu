@@ -1305,6 +1305,17 @@ void Batch::precond32(const Ti *r, Ti *z, const KState *stp) {
     const int n = h.n;
     Ti *y = v32[10].as<Ti>();
     const double fb = (4.0 + v) * h.Lf.nnz + 4.0 * (n + 1) + 2.0 * v * n;
+    if (h.tile_ok(h.Lf, h.Ltb, v)) {
+        h.timed(PC_FWD, fb, [&] {
+            sweep_tile<Ti>(h.Lf, L32.as<Ti>(), SW_FWD_DIV, r, nullptr, invL32_lev.as<Ti>(), mix_epoch, y, nullptr,
+                           h.ticket(), stp, h.err(), s);
+        });
+        h.timed(PC_BWD, fb + v * n, [&] {
+            sweep_tile<Ti>(h.Ltb, Lt32.as<Ti>(), SW_BWD_IC, nullptr, y, D32_lev.as<Ti>(), mix_epoch, z, nullptr,
+                           h.ticket() + 1, stp, h.err(), s);
+        });
+        return;
+    }
     if (h.push_ok(v)) {
         h.timed(PC_FWD, fb, [&] {
             sweep_push<Ti>(h.Lf, L32.as<Ti>(), SW_FWD_DIV, r, invL32_lev.as<Ti>(), mix_epoch, y, stp, h.err(), s);

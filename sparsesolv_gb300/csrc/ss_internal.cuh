@@ -8,6 +8,7 @@
 
 #include "ss_common.cuh"
 #include "ss_push_plan.hpp"
+#include "ss_tile_plan.hpp"
 
 namespace ssg {
 
@@ -81,6 +82,19 @@ struct PushPlan {
     unsigned long long key_epoch = ~0ull;
 };
 
+// ---------------------------------------------------------------- tile sweep plan (ss_tile.cu)
+struct TilePlan {
+    bool ready = false, failed = false;
+    int n = -1, nnz = -1, nlev = -1;  // shape of the triangle the plan was made for
+    int T = 0, lanes = 0;             // tiles; how rows are summed
+    TileLayout lay{};
+    DBuf tiles, groups, halo, rel;    // ss_tile_plan.hpp
+    DBuf rec, dval, dlv;              // the records; values refilled when the factor's values change
+    int key_fill = -1;
+    const void *key_val = nullptr, *key_lv = nullptr;
+    unsigned long long key_epoch = ~0ull;
+};
+
 // ---------------------------------------------------------------- level-scheduled triangle
 // One triangular factor in the layout the sweeps stream: rows in level order
 // (level, then row id), each row's entries contiguous and in the original
@@ -101,6 +115,7 @@ struct Tri {
     DBuf cl_code;                // per level-ordered entry: row id, or -1 - (owner << 20 | ring slot)
     DBuf cl_tab;                 // per (level, CTA): rows [rs, re) and entries [e0, e1) of the chunk
     PushPlan push[3];            // push sweep plans (ss_push.cu), one per value size: 4, 8, 16 bytes
+    TilePlan tile[3];            // tile sweep plans (ss_tile.cu), likewise
 };
 
 // ss_levels.cu
@@ -186,6 +201,15 @@ bool push_plan(Tri *const *tris, int count, size_t elem_bytes, cudaStream_t s);
 template <typename T>
 void sweep_push(Tri &tri, const T *val, int mode, const T *rhs, const T *lvec, unsigned long long epoch, T *out,
                 const KState *st, int *err, cudaStream_t s);
+
+// ss_tile.cu: whole-GPU tile sweeps (all modes; lvec: 1/diagonal, or D for SW_BWD_IC, per level-ordered row)
+// plan once per pattern and value size; false when a record does not fit (then another sweep serves)
+// lanes: 0 for real values, 4 or 8 for complex ones (the cluster sweep's lanes a row, and its bits)
+bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s);
+// epoch as for sweep_push; ticket: one int, reset here
+template <typename T>
+void sweep_tile(Tri &tri, const T *val, int mode, const T *rhs, const T *aux, const T *lvec, unsigned long long epoch,
+                T *out, T *out2, int *ticket, const KState *st, int *err, cudaStream_t s);
 
 // ss_spmv_vec.cu -- see the Krylov state there
 struct KState;

@@ -390,6 +390,12 @@ void build_tri(Tri &T, int n, int nnz, const int *rp, const int *ci, const int *
         P.key_val = P.key_lv = nullptr;
         P.key_epoch = ~0ull;
     }
+    for (TilePlan &P : T.tile) {
+        P.ready = P.failed = false;
+        P.n = P.nnz = P.nlev = -1;
+        P.key_val = P.key_lv = nullptr;
+        P.key_epoch = ~0ull;
+    }
     T.level.ensure(sizeof(int) * (size_t)n);
     T.perm.ensure(sizeof(int) * (size_t)n);
     T.ipos.ensure(sizeof(int) * (size_t)n);

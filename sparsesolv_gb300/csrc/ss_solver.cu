@@ -333,6 +333,7 @@ void Handle::ensure_sgs() {
     invU_lev.ensure(sizeof(T) * (size_t)(n + 1));
     gather_values<T>(Lf.perm.as<int>(), invC.as<T>(), invC_lev.as<T>(), n, stream);
     gather_values<T>(Ub.perm.as<int>(), invU.as<T>(), invU_lev.as<T>(), n, stream);
+    ++fac_epoch;
     sgs_valid = true;
     sgs_version = version;
 }
@@ -385,11 +386,34 @@ bool Handle::push_ok(size_t elem) {
     return push_plan(pair, 2, elem, stream);
 }
 
+// the whole-GPU tile sweeps (every mode, with the reciprocal diagonal): the automatic choice
+// where the levels are narrow enough that latency sets the pace and the plans fit. Complex
+// rows are summed as the one-cluster sweep they replace does, at its lanes a row.
+bool Handle::tile_ok(Tri &a, Tri &b, size_t elem) {
+    if (!use_inv_diag || sweep_mode != 0 || !push_auto || a.n == 0) return false;
+    const int lanes = vtype == SSG_COMPLEX ? cl_group : 0;
+    if (lanes > 8) return false;
+    for (const Tri *t : {&a, &b})
+        if ((double)t->n > kAutoClusterRowsPerLevel * (double)t->nlev) return false;
+    return tile_plan(a, elem, lanes, stream) && tile_plan(b, elem, lanes, stream);
+}
+
 // z = (L D L^T)^{-1} r using vec[10] as the forward result
 template <typename T>
 void Handle::apply_precond(const T *d_r, T *d_z, const KState *stp) {
     T *y = vec[10].as<T>();
     const size_t v = sizeof(T);
+    if (tile_ok(Lf, Ltb, v)) {
+        timed(PC_FWD, tri_bytes(Lf, v, 2), [&] {
+            sweep_tile<T>(Lf, Lval.as<T>(), SW_FWD_DIV, d_r, nullptr, invL_lev.as<T>(), fac_epoch, y, nullptr, ticket(),
+                          stp, err(), stream);
+        });
+        timed(PC_BWD, tri_bytes(Ltb, v, 3), [&] {
+            sweep_tile<T>(Ltb, Ltval.as<T>(), SW_BWD_IC, nullptr, y, D_lev.as<T>(), fac_epoch, d_z, nullptr,
+                          ticket() + 1, stp, err(), stream);
+        });
+        return;
+    }
     if (push_ok(v)) {
         timed(PC_FWD, tri_bytes(Lf, v, 2), [&] {
             sweep_push<T>(Lf, Lval.as<T>(), SW_FWD_DIV, d_r, invL_lev.as<T>(), fac_epoch, y, stp, err(), stream);
@@ -493,7 +517,10 @@ int Handle::solve(int method, double conv_cri, int max_ite, double normB, const 
     }
     if (sgs && n) {
         // rd = C^{-1} r (src/MatSolverMRTR_SGSver.cpp:118-132)
-        if (cluster_ok(Lf, sizeof(T), true)) {
+        if (tile_ok(Lf, Ub, sizeof(T))) {
+            sweep_tile<T>(Lf, Cval.as<T>(), SW_FWD_DIV, r, nullptr, invC_lev.as<T>(), fac_epoch, t1, nullptr, ticket(),
+                          nullptr, err(), s);
+        } else if (cluster_ok(Lf, sizeof(T), true)) {
             sweep_cluster<T>(Lf, Cval.as<T>(), SW_FWD_DIV, r, nullptr, use_inv_diag ? invC_lev.as<T>() : nullptr, t1,
                              nullptr, nullptr, cl_group, err(), s);
         } else {
@@ -580,7 +607,8 @@ int Handle::solve(int method, double conv_cri, int max_ite, double normB, const 
     const double nv = (double)vb * n;
     const double spmv_bytes = (4.0 + vb) * nnz + 4.0 * (n + 1) + 2.0 * nv;
     int iter_no = 0;
-    const bool sgs_cluster = sgs && cluster_ok(Ub, sizeof(T), false) && cluster_ok(Lf, sizeof(T), false);
+    const bool sgs_tile = sgs && tile_ok(Lf, Ub, sizeof(T));
+    const bool sgs_cluster = sgs && !sgs_tile && cluster_ok(Ub, sizeof(T), false) && cluster_ok(Lf, sizeof(T), false);
     auto one_iteration = [&]() {
         prof.iter = ++iter_no;
         prof.pre = true;
@@ -603,7 +631,16 @@ int Handle::solve(int method, double conv_cri, int max_ite, double normB, const 
             timed(PC_VEC, 5 * nv, [&] { mrtr_zu<T>(n, st, z, w, u, s); });
         } else {
             // u = U^{-1} rd ; ARd = u + C^{-1}(rd - u)  (src/MatSolverMRTR_SGSver.cpp:184-189)
-            if (sgs_cluster) {
+            if (sgs_tile) {
+                timed(PC_BWD, tri_bytes(Ub, vb, 2), [&] {
+                    sweep_tile<T>(Ub, Uval.as<T>(), SW_BWD_DIV, r, nullptr, invU_lev.as<T>(), fac_epoch, u, nullptr,
+                                  ticket(), st, err(), s);
+                });
+                timed(PC_FWD, tri_bytes(Lf, vb, 4), [&] {
+                    sweep_tile<T>(Lf, Cval.as<T>(), SW_FWD_EIS, r, u, invC_lev.as<T>(), fac_epoch, t1, w, ticket() + 1,
+                                  st, err(), s);
+                });
+            } else if (sgs_cluster) {
                 timed(PC_BWD, tri_bytes(Ub, vb, 2), [&] {
                     sweep_cluster<T>(Ub, Uval.as<T>(), SW_BWD_DIV, r, nullptr,
                                      use_inv_diag ? invU_lev.as<T>() : nullptr, u, nullptr, st, cl_group, err(), s);
@@ -692,7 +729,10 @@ Handle::TuneChoice Handle::autotune(bool keep_group, bool with_push) {
         }
     // the push sweep sums each row in dependency-level order, not by lanes: a candidate
     // only when the summation order is free to change
-    if (!keep_group && with_push) cand.push_back({4, 1, 0, 0.0});
+    if (!keep_group && with_push) {
+        cand.push_back({4, 1, 0, 0.0});
+        cand.push_back({0, 4, 0, 0.0});  // the automatic choice: the tile sweep
+    }
     const TuneChoice before{sweep_mode, swcfg.group, swcfg.cta_per_sm, 0.0};
     const int cl_before = cl_group;
     const bool prof_on = prof.on;

@@ -124,6 +124,7 @@ struct Handle {
     // ic: an IC sweep (the only kind the neighbour-synchronised plan serves)
     bool cluster_ok(Tri &t, size_t elem, bool ic);
     bool push_ok(size_t elem);  // both triangles of the IC pair
+    bool tile_ok(Tri &a, Tri &b, size_t elem);  // the whole-GPU tile sweeps serve both triangles
     // the automatic mode may take the push sweep (off in the standalone batches: their
     // instances' bits must not depend on which schedule a batch's size leads to, and the
     // lane-summed schedules give the same bits at the same lanes a row)

@@ -1,0 +1,639 @@
+// ss_tile.cu -- whole-GPU tile sweeps for every triangular solve of the solvers:
+// the IC pair of MatSolverBase::IC_frbc_process (src/MatSolverBase.cpp:177-231),
+// fr_process / bc_process (:243-327) and the Eisenstat sweep of
+// MatSolverMRTR_SGSver.cpp:187-189.
+//
+// A sweep is bound by its dependency levels, not by bytes. The schedule
+// (ss_tile_plan.hpp) cuts the rows into tiles of consecutive rows; a CTA owns a
+// tile, so all but the tile borders of a dependency path stay inside one SM, and
+// because tiles only depend on lower tiles, the latency of a border is paid once
+// per border and not once per level.
+//
+// A CTA claims tiles in order through a ticket (every wait is on a tile some
+// running CTA holds) and runs three kinds of warps:
+//   * compute warps take the tile's groups round robin (group g: warp g % TS_W),
+//     sum, write the values to the own ring, publish their progress and store the
+//     values to memory;
+//   * receiver warps bring the halo in, 32 values a chunk: each lane polls the
+//     output vector for one value (a sentinel marks the unsolved) and puts it into
+//     the halo ring; the count of values here, in list order, is published;
+//   * one warp stages the groups' records with bulk copies as ring space frees.
+// Waits inside a CTA are one load of the progress words and one vote.
+// Values go between CTAs through the output vector alone: an aligned 4- or 8-byte
+// store is single-copy atomic, so a value is its own flag and no fence is needed.
+//
+// What bounds it: the chain of dependency levels (1,410 forward at 80^3), not bytes
+// (1 % of HBM) and not yet FP64: an FP64 instruction holds its warp for 64 cycles
+// and an SM issues one in 19, so a group's 12-15 instructions set the split of the
+// sums. Measured on a GB300, microseconds a sweep (forward / backward), with the
+// one-cluster schedules this replaces as the automatic choice in brackets:
+//   curl-curl, real:  10^3  54 / 55 [221 / 222], 20^3 124 / 126 [496 / 501],
+//                     41^3 371 / 359 [1,095 / 1,090], 80^3 1,079 / 1,023 [2,237 / 2,195] (push)
+//   SGS pair, 48^3:   490 / 483 [1,834 / 1,810] (lockstep)
+//   eddy currents:    33^3 727 / 906 [1,638 / 1,525], 60^3 1,526 / 1,839 [3,616 / 3,338] (lockstep)
+//   FP32, 44^3:       206 / 210 [504 / 498] (push)
+//
+// Every wait is bounded (the handle's spin limit) and ends early when the error
+// word is set; the CTA then drains its copies and leaves.
+#include <algorithm>
+
+#include "sparsesolv_gb300.h"
+#include "ss_internal.cuh"
+#include "ss_krylov.cuh"
+
+namespace ssg {
+
+// ---------------------------------------------------------------- device helpers
+__device__ __forceinline__ void tl_mbar_init(unsigned a, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
+}
+__device__ __forceinline__ void tl_mbar_inval(unsigned a) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(a) : "memory");
+}
+__device__ __forceinline__ void tl_mbar_expect(unsigned a, unsigned tx) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(tx) : "memory");
+}
+__device__ __forceinline__ bool tl_mbar_test(unsigned a, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(a), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void tl_bulk_g2s(unsigned dst, const void *src, unsigned bytes, unsigned mbar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(mbar)
+                 : "memory");
+}
+__device__ __forceinline__ void tl_st_release(unsigned a, int v) {
+    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ int tl_ld_acquire(unsigned a) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+// one value of the output vector, written by any CTA: false while unsolved
+__device__ __forceinline__ bool tl_take(const double *p, double &v) {
+    v = ld_vol(p);
+    return !is_sent(v);
+}
+__device__ __forceinline__ bool tl_take(const float *p, float &v) {
+    v = ld_vol(p);
+    return !is_sent(v);
+}
+__device__ __forceinline__ bool tl_take(const cplx *p, cplx &v) {
+    v.x = ld_vol(&p->x);
+    v.y = ld_vol(&p->y);
+    return !is_sent(v.x) && !is_sent(v.y);
+}
+__device__ __forceinline__ bool tl_take(const cplxf *p, cplxf &v) {
+    v.x = ld_vol(&p->x);
+    v.y = ld_vol(&p->y);
+    return !is_sent(v.x) && !is_sent(v.y);
+}
+__device__ __forceinline__ void tl_give(double *p, double v) { st_vol(p, unsent(v)); }
+__device__ __forceinline__ void tl_give(float *p, float v) { st_vol(p, unsent(v)); }
+__device__ __forceinline__ void tl_give(cplx *p, cplx v) {
+    st_vol(&p->x, unsent(v.x));
+    st_vol(&p->y, unsent(v.y));
+}
+__device__ __forceinline__ void tl_give(cplxf *p, cplxf v) {
+    st_vol(&p->x, unsent(v.x));
+    st_vol(&p->y, unsent(v.y));
+}
+
+// a warp that tests a staged group's barrier has itself taken the group staged there before, so the parity is unambiguous
+static_assert(TS_NM % TS_W == 0, "groups of one barrier belong to one warp");
+static_assert(TS_TAILS == 2 && TS_W < 32, "the stages and progress words below");
+
+// one lane's four values of a block of columns (ts_col)
+__device__ __forceinline__ void tl_vals(const double *b, int lane, double (&v)[4]) {
+    const double2 p = ((const double2 *)b)[lane], q = ((const double2 *)b)[32 + lane];
+    v[0] = p.x, v[1] = p.y, v[2] = q.x, v[3] = q.y;
+}
+__device__ __forceinline__ void tl_vals(const float *b, int lane, float (&v)[4]) {
+    const float4 p = ((const float4 *)b)[lane];
+    v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = p.w;
+}
+__device__ __forceinline__ void tl_vals(const cplx *b, int lane, cplx (&v)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double2 p = ((const double2 *)b)[32 * q + lane];
+        v[q] = {p.x, p.y};
+    }
+}
+__device__ __forceinline__ void tl_vals(const cplxf *b, int lane, cplxf (&v)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; q += 2) {
+        const float4 p = ((const float4 *)b)[16 * q + lane];
+        v[q] = {p.x, p.y};
+        v[q + 1] = {p.z, p.w};
+    }
+}
+
+struct TileArgs {
+    int T;
+    const int4 *tiles, *groups;
+    const int *halo, *rel;
+    const unsigned char *rec;
+    const void *rhs, *aux;
+    void *out, *out2;
+    int *ticket;   // zero at launch
+    const KState *st;
+    int *err;
+    TileLayout L;
+};
+
+// the time limit of a wait, looked at every so many polls
+struct Bound {
+    int *err;
+    unsigned long long lim, t0 = 0;
+    unsigned polls = 0;
+    __device__ Bound(int *e, unsigned long long l) : err(e), lim(l) {}
+    // true: give up
+    __device__ __forceinline__ bool spent(unsigned mask) {
+        if ((++polls & mask) != 0) return false;
+        if (*(volatile int *)err) return true;
+        const unsigned long long t = gtimer();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > lim) {
+            atomicExch(err, ERR_TIMEOUT);
+            return true;
+        }
+        return false;
+    }
+};
+
+// LANES: 0 sums by age, 4 or 8 by lanes (ss_tile_plan.hpp)
+template <typename T, int MODE, int LANES>
+__global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
+    if (a.st && !a.st->active) return;
+    extern __shared__ __align__(16) unsigned char tl_smem[];
+    __shared__ int s_tile;
+    const TileLayout &L = a.L;
+    const unsigned sbase = (unsigned)__cvta_generic_to_shared(tl_smem);
+    T *X = (T *)(tl_smem + L.o_x);
+    int *place = (int *)(tl_smem + L.o_place);  // record ring offsets / 16 of the staged groups
+    const unsigned full = sbase + L.o_full, prog = sbase + L.o_prog;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const T *rhs = (const T *)a.rhs, *aux = (const T *)a.aux;
+    T *out = (T *)a.out, *out2 = (T *)a.out2;
+    const unsigned long long lim = spin_limit_ns(a.err);
+    constexpr int EB = (int)sizeof(T);
+    bool bad = false;
+
+    if (tid == 0) X[L.S_own + L.S_halo] = Sc<T>::zero();
+    for (;;) {
+        // ---- next tile
+        if (tid == 0) s_tile = atomicAdd(a.ticket, 1);
+        if (tid < TS_NM) tl_mbar_init(full + 8u * tid, 1);
+        if (tid < 32) ((volatile int *)(tl_smem + L.o_prog))[tid] = tid < TS_W ? tid : 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncthreads();
+        const int tile = s_tile;
+        if (tile >= a.T) break;
+        const int4 td = a.tiles[tile];
+        const int ng = td.y, nch = td.w;
+        int issued = 0;  // groups staged
+
+        // own groups up to og are done and h halo values are here
+        auto ready = [&](int og, int h) {
+            const int want = lane < TS_W ? og + 1 : lane == TS_W ? h : 0;
+            return __all_sync(0xffffffffu, tl_ld_acquire(prog + 4u * lane) >= want) != 0;
+        };
+        auto wait_for = [&](int og, int h) {
+            if (ready(og, h)) return;
+            Bound b(a.err, lim);
+            while (!(ready(og, h) || ready(og, h) || ready(og, h)))
+                if (__any_sync(0xffffffffu, b.spent(255))) {
+                    bad = true;
+                    return;
+                }
+        };
+        // group g's record, once staged; null: give up
+        auto record = [&](int g) -> const unsigned char * {
+            const unsigned bar = full + 8u * (g % TS_NM);
+            const unsigned par = (unsigned)((g / TS_NM) & 1);
+            if (!tl_mbar_test(bar, par)) {
+                Bound b(a.err, lim);
+                while (!tl_mbar_test(bar, par))
+                    if (b.spent(255)) {
+                        bad = true;
+                        break;
+                    }
+            }
+            bad = __any_sync(0xffffffffu, bad);
+            return bad ? nullptr : tl_smem + L.o_rec + 16 * place[g % TS_NM];
+        };
+
+        if (warp < TS_W) {
+            // ------------------------------------------------ compute warps
+            for (int g = warp; g < ng; g += TS_W) {
+                const unsigned char *rec = record(g);
+                if (!rec) break;
+                const int4 *hd = (const int4 *)rec;
+                const int4 h0 = hd[0], nd = hd[1], of = hd[3];
+                const int cnt = h0.x & 0xff, lg = (h0.x >> 8) & 0xff;
+                const int nb = h0.y & 0xffff;
+                const int *cfar = (h0.y >> 16) ? (const int *)(rec + 16 * of.z) : nullptr;
+                const int2 *need = (const int2 *)(rec + 64);
+                const T *v = (const T *)(rec + 16 * (of.x & 0xffff));
+                // a column's value: from the rings, or from memory where its slot is reused too early
+                auto value = [&](int code, const int *far_row) -> T {
+                    if (code != TS_FAR) return X[code];
+                    T x = Sc<T>::zero();
+                    if (!tl_take(out + *far_row, x)) {
+                        Bound b(a.err, lim);
+                        while (!tl_take(out + *far_row, x))
+                            if (b.spent(63)) {
+                                bad = true;
+                                break;
+                            }
+                    }
+                    return x;
+                };
+                T res = Sc<T>::zero(), u0 = res;
+                int row = 0;
+                bool lead;  // this lane has the row's result
+                if (LANES > 0) {
+                    const int r = lane / LANES;
+                    lead = lane % LANES == 0 && r < cnt;
+                    T b0 = Sc<T>::zero(), lv = b0;
+                    if (lead) {
+                        row = ((const int *)(rec + 16 * (of.w & 0xffff)))[r];
+                        lv = ((const T *)(rec + 16 * ((unsigned)of.w >> 16)))[r];
+                        if (MODE != SW_BWD_IC) b0 = rhs[row];
+                        if (MODE == SW_BWD_IC || MODE == SW_FWD_EIS) u0 = aux[row];
+                    }
+                    // the arithmetic of k_sweep: the forward right-hand side starts lane 0's sum, the IC pair's values
+                    // come negated
+                    T acc = MODE == SW_FWD_DIV ? b0 : Sc<T>::zero();
+                    const unsigned short *c = (const unsigned short *)(rec + 16 * (of.y & 0xffff)) + lane;
+                    v += lane;
+#pragma unroll 1
+                    for (int k = 0; k < nb; ++k) {
+                        const int2 w = need[k];
+                        const int cc = c[32 * k];
+                        const T vv = v[32 * k];
+                        wait_for(w.x, w.y);
+                        acc = madd(acc, vv, cfar ? value(cc, cfar + 32 * k + lane) : X[cc]);
+                    }
+                    if (cfar) __syncwarp();
+#pragma unroll
+                    for (int m = LANES / 2; m >= 1; m >>= 1) acc = acc + Sc<T>::shfl_xor(acc, m);
+                    if (MODE == SW_BWD_IC) res = madd(u0, lv, acc);
+                    else if (MODE == SW_FWD_DIV) res = acc * lv;
+                    else if (MODE == SW_FWD_EIS) res = ((b0 - u0) - acc) * lv;
+                    else res = (b0 - acc) * lv;
+                    wait_for(nd.z, nd.w);  // the own-ring slots are free
+                    if (lead) X[(h0.z + r) & (L.S_own - 1)] = res;
+                } else {
+                    const int k1 = (h0.x >> 16) & 15, k2 = (h0.x >> 20) & 15;
+                    lead = lane < cnt;  // lane r has row r outside the columns
+                    // what the row starts from: on its way while the first block waits
+                    T b0 = Sc<T>::zero(), lv = b0;
+                    if (lead) {
+                        row = ((const int *)(rec + 16 * (of.w & 0xffff)))[lane];
+                        if (MODE != SW_BWD_IC) {
+                            lv = ((const T *)(rec + 16 * ((unsigned)of.w >> 16)))[lane];
+                            b0 = rhs[row];
+                        }
+                        if (MODE == SW_BWD_IC || MODE == SW_FWD_EIS) u0 = aux[row];
+                    }
+                    // ---- columns: one or two lanes a row, the even and the odd columns in two sums
+                    T s0 = Sc<T>::zero(), s1 = s0;
+                    const ushort4 *c = (const ushort4 *)(rec + 16 * (of.y & 0xffff)) + lane;
+                    int skip = 4 - h0.w;
+#pragma unroll 1
+                    for (int k = 0; k < nb; ++k) {
+                        const int2 w = need[k];
+                        const ushort4 cc = c[32 * k];
+                        T vv[4], x0, x1, x2, x3;
+                        tl_vals(v + 128 * k, lane, vv);
+                        wait_for(w.x, w.y);
+                        if (!cfar) {
+                            x0 = X[cc.x], x1 = X[cc.y], x2 = X[cc.z], x3 = X[cc.w];
+                        } else {
+                            const int *f = cfar + 128 * k + 4 * lane;
+                            x0 = value(cc.x, f), x1 = value(cc.y, f + 1), x2 = value(cc.z, f + 2), x3 = value(cc.w, f + 3);
+                            __syncwarp();
+                        }
+                        // jumps, not predicates, past the first block's empty columns: a multiply-add costs the FP64
+                        // latency whether or not it runs
+                        if (lg) {
+                            switch (skip) {
+                                case 0: s0 = madd(s0, vv[0], x0); [[fallthrough]];
+                                case 1: s0 = madd(s0, vv[1], x1); [[fallthrough]];
+                                case 2: s0 = madd(s0, vv[2], x2); [[fallthrough]];
+                                default: s0 = madd(s0, vv[3], x3);
+                            }
+                        } else {
+                            switch (skip) {
+                                case 0: s0 = madd(s0, vv[0], x0); [[fallthrough]];
+                                case 1: s1 = madd(s1, vv[1], x1); [[fallthrough]];
+                                case 2: s0 = madd(s0, vv[2], x2); [[fallthrough]];
+                                default: s1 = madd(s1, vv[3], x3);
+                            }
+                        }
+                        skip = 0;
+                    }
+                    if (nb > 0) {
+                        if (lg) {
+                            s0 = s0 + Sc<T>::shfl_xor(s0, 1);
+                            s0 = Sc<T>::shfl(s0, (2 * lane) & 31);  // lane r takes row r's sum
+                        } else {
+                            s0 = s0 + s1;
+                        }
+                    }
+                    if (MODE == SW_BWD_IC) res = u0 + s0;
+                    else if (MODE == SW_FWD_EIS) res = madd(s0, b0 - u0, lv);
+                    else res = madd(s0, b0, lv);
+                    // ---- tails: one lane a row; the first two values and codes of both stages ahead of the waits
+                    const T *v1 = (const T *)(rec + 16 * ((unsigned)of.x >> 16)) + lane, *v2 = v1 + 32 * k1;
+                    const unsigned short *c1 = (const unsigned short *)(rec + 16 * ((unsigned)of.y >> 16)) + lane,
+                                         *c2 = c1 + 32 * k1;
+                    // reads past a stage's entries stay inside the shared memory (tile_layout) and are not used
+                    const T va = v1[0], vb = v1[32], wa = v2[0], wb = v2[32];
+                    const int ca = c1[0], cb = c1[32], da = c2[0], db = c2[32];
+                    if (k1 > 0) {
+                        wait_for(nd.x, nd.y);
+                        if (k1 > 1) {
+                            const T xa = X[ca], xb = X[cb];
+                            res = madd(res, va, xa);
+                            res = madd(res, vb, xb);
+#pragma unroll 1
+                            for (int k = 2; k < k1; ++k) res = madd(res, v1[32 * k], X[c1[32 * k]]);
+                        } else {
+                            res = madd(res, va, X[ca]);
+                        }
+                    }
+                    wait_for(nd.z, nd.w);
+                    if (k2 > 0) {
+                        if (k2 > 1) {
+                            const T xa = X[da], xb = X[db];
+                            res = madd(res, wa, xa);
+                            res = madd(res, wb, xb);
+#pragma unroll 1
+                            for (int k = 2; k < k2; ++k) res = madd(res, v2[32 * k], X[c2[32 * k]]);
+                        } else {
+                            res = madd(res, wa, X[da]);
+                        }
+                    }
+                    if (lead) X[(h0.z + lane) & (L.S_own - 1)] = res;
+                }
+                __syncwarp();
+                if (lane == 0) tl_st_release(prog + 4u * warp, g + TS_W);
+                if (lead) {
+                    tl_give(out + row, res);
+                    if (MODE == SW_FWD_EIS) out2[row] = res + u0;
+                }
+            }
+        } else if (warp < TS_W + TS_R) {
+            // ------------------------------------------------ receiver warps
+            // chunk ch (32 values) is this warp's for ch % TS_R == me; a value counts as soon as it and all before it are here
+            const int me = warp - TS_W;
+            const unsigned count = prog + 4u * TS_W;
+            const int *hl = a.halo + 32ll * td.z;
+            int j = me < nch ? hl[32 * me + lane] : -1;
+            int rel = me < nch ? a.rel[td.z + me] : -1;
+            for (int ch = me; ch < nch; ch += TS_R) {
+                const int jn = ch + TS_R < nch ? hl[32 * (ch + TS_R) + lane] : -1;
+                const int reln = ch + TS_R < nch ? a.rel[td.z + ch + TS_R] : -1;
+                // the slots' previous values are dead (they are, long since, unless the halo ring is full)
+                if (rel >= 0) wait_for(rel, 0);
+                bool have = j < 0, head = false;
+                int told = 0, tries = 0;
+                Bound b(a.err, lim);
+                while (!bad) {
+                    T x;
+                    if (!have && tl_take(out + j, x)) {
+                        X[L.S_own + ((32 * ch + lane) & (L.S_halo - 1))] = x;
+                        have = true;
+                    }
+                    const unsigned miss = ~__ballot_sync(0xffffffffu, have);
+                    if (!head) head = __all_sync(0xffffffffu, tl_ld_acquire(count) >= 32 * ch);
+                    const int now = miss ? __ffs(miss) - 1 : 32;
+                    if (head && now > told) {
+                        __syncwarp();
+                        if (lane == 0) tl_st_release(count, 32 * ch + now);
+                        told = now;
+                    }
+                    if (told == 32) break;
+                    if (__any_sync(0xffffffffu, b.spent(63))) bad = true;
+                    // far ahead of the producers: poll gently
+                    if (++tries > 16) __nanosleep(100);
+                }
+                if (bad) break;
+                j = jn;
+                rel = reln;
+            }
+        } else {
+            // ------------------------------------------------ staging warp
+            for (int g0 = 0; g0 < ng && !bad; g0 += 32) {
+                const int4 m = a.groups[td.x + min(g0 + lane, ng - 1)];
+                for (int q = 0; q < 32 && g0 + q < ng; ++q) {
+                    const int src = __shfl_sync(0xffffffffu, m.x, q), n16 = __shfl_sync(0xffffffffu, m.y, q);
+                    const int dst = __shfl_sync(0xffffffffu, m.z, q), need = __shfl_sync(0xffffffffu, m.w, q);
+                    if (need >= 0) wait_for(need, 0);
+                    if (bad) break;
+                    if (lane == 0) {
+                        const unsigned bar = full + 8u * ((g0 + q) % TS_NM);
+                        place[(g0 + q) % TS_NM] = dst;  // the arrival below releases it to the group's warp
+                        tl_mbar_expect(bar, 16u * (unsigned)n16);
+                        tl_bulk_g2s(sbase + L.o_rec + 16u * (unsigned)dst, a.rec + 16ll * src, 16u * (unsigned)n16, bar);
+                    }
+                    issued = g0 + q + 1;
+                }
+            }
+        }
+        if (__syncthreads_or(bad)) {
+            // copies in flight land before the shared memory goes away (bounded)
+            if (warp == TS_W + TS_R && lane == 0)
+                for (int g = max(0, issued - TS_NM); g < issued; ++g) {
+                    const unsigned long long t0 = gtimer();
+                    while (!tl_mbar_test(full + 8u * (g % TS_NM), (unsigned)((g / TS_NM) & 1)) &&
+                           gtimer() - t0 < 1000000ull) {
+                    }
+                }
+            return;
+        }
+        if (tid < TS_NM) tl_mbar_inval(full + 8u * tid);
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------- record values (once per factor)
+// by age rec[dval[k]] = -val[k] * lvec[t]; by lanes val[k], negated for the IC pair; rec[dlv[t]] = lvec[t]
+enum : int { TF_SCALED = 0, TF_PLAIN = 1, TF_NEG = 2 };
+template <typename T, int FILL>
+__global__ void k_tile_fill(int n, const int *prp, const int *dval, const int *dlv, const T *val, const T *lvec, T *rec) {
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, q = threadIdx.x & 3;
+    if (t >= n) return;
+    const T lv = lvec[t];
+    if (q == 0) rec[dlv[t]] = lv;
+    for (int k = prp[t] + q; k < prp[t + 1]; k += 4) {
+        const int d = dval[k];
+        if (d >= 0) rec[d] = FILL == TF_SCALED ? -(val[k] * lv) : FILL == TF_NEG ? -val[k] : val[k];
+    }
+}
+
+// the output vector unsolved, the ticket back at tile 0
+template <typename W>
+__global__ void k_tile_arm(W *p, size_t words, int *ticket, const KState *st) {
+    if (st && !st->active) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x)
+        p[i] = (W)~(W)0;
+}
+
+static int tile_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        sms = v > 0 ? v : 1;
+    }
+    return sms;
+}
+
+// The plan: once per pattern and value size, on the host (ss_tile_plan.cpp)
+bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s) {
+    const int elem = (int)elem_bytes, slot = elem == 4 ? 0 : elem == 8 ? 1 : 2;
+    TilePlan &P = T.tile[slot];
+    if (P.n != T.n || P.nnz != T.nnz || P.nlev != T.nlev || P.lanes != lanes) {
+        P.ready = P.failed = false;
+        P.lanes = lanes;
+        P.n = T.n;
+        P.nnz = T.nnz;
+        P.nlev = T.nlev;
+    }
+    if (P.ready) return true;
+    if (P.failed || T.n == 0) return false;
+    std::vector<int> prp(T.n + 1), pci(T.nnz), ipos(T.n), level(T.n);
+    SSG_CUDA(cudaMemcpyAsync(prp.data(), T.prp.p, sizeof(int) * (T.n + 1), cudaMemcpyDeviceToHost, s));
+    SSG_CUDA(cudaMemcpyAsync(pci.data(), T.pci.p, sizeof(int) * (size_t)T.nnz, cudaMemcpyDeviceToHost, s));
+    SSG_CUDA(cudaMemcpyAsync(ipos.data(), T.ipos.p, sizeof(int) * T.n, cudaMemcpyDeviceToHost, s));
+    SSG_CUDA(cudaMemcpyAsync(level.data(), T.level.p, sizeof(int) * T.n, cudaMemcpyDeviceToHost, s));
+    SSG_CUDA(cudaStreamSynchronize(s));
+    const TilePlanHost H =
+        tile_plan_host(T.n, T.nlev, prp.data(), pci.data(), ipos.data(), level.data(), T.lower, elem, lanes, 0);
+    if (!H.ok) {
+        P.failed = true;
+        return false;
+    }
+    auto put = [&](DBuf &d, const std::vector<int> &h) {
+        d.ensure(sizeof(int) * (h.size() + 4));
+        if (!h.empty()) SSG_CUDA(cudaMemcpyAsync(d.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, s));
+    };
+    put(P.tiles, H.tiles);
+    put(P.groups, H.groups);
+    put(P.halo, H.halo);
+    put(P.rel, H.rel);
+    put(P.dval, H.dval);
+    put(P.dlv, H.dlv);
+    P.rec.ensure((size_t)H.rec_bytes + 16);
+    for (int t = 0; t < H.T; ++t)
+        if (!H.rec[t].empty())
+            SSG_CUDA(cudaMemcpyAsync(P.rec.as<unsigned char>() + H.rec_off[t], H.rec[t].data(), H.rec[t].size(),
+                                     cudaMemcpyHostToDevice, s));
+    SSG_CUDA(cudaStreamSynchronize(s));
+    P.lay = H.lay;
+    P.T = H.T;
+    P.key_val = P.key_lv = nullptr;
+    P.key_epoch = ~0ull;
+    P.ready = true;
+    return true;
+}
+
+template <typename T>
+void sweep_tile(Tri &tri, const T *val, int mode, const T *rhs, const T *aux, const T *lvec, unsigned long long epoch,
+                T *out, T *out2, int *ticket, const KState *st, int *err, cudaStream_t s) {
+    TilePlan &P = tri.tile[sizeof(T) == 4 ? 0 : sizeof(T) == 8 ? 1 : 2];
+    if (tri.n == 0) return;
+    if (!P.ready || P.n != tri.n || P.nnz != tri.nnz || P.nlev != tri.nlev)
+        throw Error{SSG_ERR_STATE, "tile sweep without a plan for this triangle"};
+    constexpr bool by_lanes = Sc<T>::is_complex;
+    const int fill = !by_lanes ? TF_SCALED : mode == SW_FWD_DIV || mode == SW_BWD_IC ? TF_NEG : TF_PLAIN;
+    if (P.key_val != val || P.key_lv != lvec || P.key_epoch != epoch || P.key_fill != fill) {
+        auto k = fill == TF_SCALED ? k_tile_fill<T, TF_SCALED> : fill == TF_NEG ? k_tile_fill<T, TF_NEG> : k_tile_fill<T, TF_PLAIN>;
+        k<<<div_up((long long)tri.n * 4, 256), 256, 0, s>>>(tri.n, tri.prp.as<int>(), P.dval.as<int>(), P.dlv.as<int>(), val,
+                                                            lvec, P.rec.as<T>());
+        SSG_LAUNCHED();
+        P.key_val = val;
+        P.key_lv = lvec;
+        P.key_epoch = epoch;
+        P.key_fill = fill;
+    }
+    {
+        using W = unsigned long long;
+        const size_t bytes = sizeof(T) * (size_t)tri.n;
+        if (bytes % 8 == 0 && ((size_t)out & 7) == 0)
+            k_tile_arm<W><<<std::min(div_up((long long)(bytes / 8), 1024), 4 * tile_sms()), 256, 0, s>>>(
+                (W *)out, bytes / 8, ticket, st);
+        else
+            k_tile_arm<unsigned><<<std::min(div_up((long long)(bytes / 4), 1024), 4 * tile_sms()), 256, 0, s>>>(
+                (unsigned *)out, bytes / 4, ticket, st);
+        SSG_LAUNCHED();
+    }
+    TileArgs a;
+    a.T = P.T;
+    a.tiles = P.tiles.as<int4>();
+    a.groups = P.groups.as<int4>();
+    a.halo = P.halo.as<int>();
+    a.rel = P.rel.as<int>();
+    a.rec = P.rec.as<unsigned char>();
+    a.rhs = rhs;
+    a.aux = aux;
+    a.out = out;
+    a.out2 = out2;
+    a.ticket = ticket;
+    a.st = st;
+    a.err = err;
+    a.L = P.lay;
+    const int grid = std::min(P.T, tile_sms());
+#define SSG_TS(M, LN)                                                                                          \
+    do {                                                                                                       \
+        auto kern = k_sweep_tile<T, M, LN>;                                                                    \
+        static bool prepared = false;                                                                          \
+        if (!prepared) {                                                                                       \
+            SSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX));    \
+            prepared = true;                                                                                   \
+        }                                                                                                      \
+        kern<<<grid, TS_THREADS, P.lay.total, s>>>(a);                                                         \
+    } while (0)
+#define SSG_TM(LN)                                                \
+    switch (mode) {                                               \
+        case SW_FWD_DIV: SSG_TS(SW_FWD_DIV, LN); break;           \
+        case SW_BWD_IC: SSG_TS(SW_BWD_IC, LN); break;             \
+        /* by age the same arithmetic on the other triangle */    \
+        case SW_BWD_DIV: SSG_TS((LN ? SW_BWD_DIV : SW_FWD_DIV), LN); break; \
+        default: SSG_TS(SW_FWD_EIS, LN); break;                   \
+    }
+    if constexpr (!by_lanes) {
+        SSG_TM(0)
+    } else if (P.lanes == 4) {
+        SSG_TM(4)
+    } else {
+        SSG_TM(8)
+    }
+#undef SSG_TM
+#undef SSG_TS
+    SSG_LAUNCHED();
+}
+
+#define SSG_INST(T)                                                                                              \
+    template void sweep_tile<T>(Tri &, const T *, int, const T *, const T *, const T *, unsigned long long, T *, \
+                                T *, int *, const KState *, int *, cudaStream_t);
+SSG_INST(double)
+SSG_INST(cplx)
+SSG_INST(float)
+SSG_INST(cplxf)
+#undef SSG_INST
+
+}  // namespace ssg

@@ -1,0 +1,429 @@
+// ss_tile_plan.cpp -- the tile sweep's schedule (ss_tile_plan.hpp says what it is, ss_tile.cu runs it).
+//
+// Tiles are planned independently of each other, on host threads; the outputs are put in tile order, so the plan does
+// not depend on the thread count (SSG_PLAN_THREADS, 1-64).
+#include "ss_tile_plan.hpp"
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <deque>
+#include <exception>
+#include <thread>
+
+namespace ssg {
+
+TileLayout tile_layout(int elem) {
+    TileLayout L{};
+    // 32 KB each for the own and the halo ring whatever the value size; the rest stages records
+    L.S_own = 32 * 1024 / elem;
+    L.S_halo = 32 * 1024 / elem;
+    int o = 0;
+    L.o_x = o;
+    o += ts_al16((L.S_own + L.S_halo + 1) * elem);
+    L.o_full = o;
+    o += 8 * TS_NM;
+    L.o_place = o;
+    o += 4 * TS_NM;
+    L.o_prog = o;  // compute warps' next groups, then the number of halo values delivered
+    o += 4 * 32;
+    L.o_rec = o;
+    // the kernel loads two tail entries of a stage ahead, whether or not it has them
+    const int slack = 64 * elem + 128;
+    L.B_rec = (TS_SMEM_MAX - o - slack) & ~15;
+    L.total = o + L.B_rec + slack;
+    return L;
+}
+
+// More tiles put fewer rows of a level on an SM, each border costs its latency once. Measured best (us a forward sweep):
+// 2,430 rows 1 tile 48, 2 tiles 51; 21,660 rows 8 tiles 116, 16 120; 196,800 rows 32-64 tiles 364, 100 375; 1,497,840 rows
+// 152 tiles 1,124, 300 1,048. 0.014 n^0.7 is 3, 15, 71 and 294.
+int tile_count(int n) {
+    const int t = (int)std::lround(0.014 * std::pow((double)n, 0.7));
+    return std::max(1, std::min(t, n));
+}
+
+namespace {
+
+struct TileOut {
+    std::vector<int> groups, halo, rel;  // ring offsets and groups relative to the tile
+    std::vector<unsigned char> rec;
+    int nfar = 0;
+    const char *why = nullptr;
+};
+
+struct Ctx {
+    int n, elem, lanes;
+    const int *prp, *pci, *ipos, *level;
+    bool lower;
+    TileLayout L;
+    int *dval, *dlv;  // element indices relative to the tile's records; made absolute afterwards
+    int row(int p) const { return lower ? p : n - 1 - p; }
+    int ord(int i) const { return lower ? i : n - 1 - i; }
+};
+
+struct Entry {
+    int lev, j, k;   // dependency level, row, index in the level-ordered triangle
+};
+
+// scratch of one planning thread
+struct Scratch {
+    std::vector<int> hpos;  // row -> halo position of the current tile, -1
+    explicit Scratch(int n) : hpos((size_t)n, -1) {}
+};
+
+void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
+    const int nr = p1 - p0, elem = C.elem;
+    const TileLayout &L = C.L;
+    // rows in (level, order), and groups of rows of one level
+    int lmin = 1 << 30, lmax = 0;
+    for (int p = p0; p < p1; ++p) {
+        const int l = C.level[C.row(p)];
+        lmin = std::min(lmin, l);
+        lmax = std::max(lmax, l);
+    }
+    std::vector<int> cnt((size_t)(lmax - lmin) + 2, 0), rows((size_t)nr), pos((size_t)nr), grp((size_t)nr);
+    for (int p = p0; p < p1; ++p) cnt[C.level[C.row(p)] - lmin + 1]++;
+    for (size_t l = 1; l < cnt.size(); ++l) cnt[l] += cnt[l - 1];
+    {
+        std::vector<int> at(cnt.begin(), cnt.end() - 1);
+        for (int p = p0; p < p1; ++p) {
+            const int q = at[C.level[C.row(p)] - lmin]++;
+            rows[q] = p;
+            pos[p - p0] = q;
+        }
+    }
+    std::vector<int> gfirst;
+    const int most = C.lanes ? 32 / C.lanes : 32;  // rows of a group
+    for (int q = 0; q < nr;) {
+        const int l = C.level[C.row(rows[q])];
+        int e = q;
+        while (e < nr && e - q < most && C.level[C.row(rows[e])] == l) ++e;
+        gfirst.push_back(q);
+        for (int k = q; k < e; ++k) grp[k] = (int)gfirst.size() - 1;
+        q = e;
+    }
+    const int ng = (int)gfirst.size();
+    gfirst.push_back(nr);
+    // halo: the rows of other tiles read here, in (level, order)
+    std::vector<int> hal;
+    for (int q = 0; q < nr; ++q) {
+        const int i = C.row(rows[q]), t = C.ipos[i];
+        for (int k = C.prp[t]; k < C.prp[t + 1]; ++k) {
+            const int j = C.pci[k];
+            if (j == i) continue;
+            if (j < 0 || j >= C.n || C.ord(j) >= C.ord(i) || C.level[j] >= C.level[i]) {
+                O.why = "an entry is not a dependency of its row";
+                for (int h : hal) S.hpos[h] = -1;
+                return;
+            }
+            if (C.ord(j) < p0 && S.hpos[j] < 0) {
+                S.hpos[j] = 0;
+                hal.push_back(j);
+            }
+        }
+    }
+    std::sort(hal.begin(), hal.end(), [&](int a, int b) {
+        return C.level[a] != C.level[b] ? C.level[a] < C.level[b] : C.ord(a) < C.ord(b);
+    });
+    const int nh = (int)hal.size(), nch = (nh + 31) / 32;
+    for (int q = 0; q < nh; ++q) S.hpos[hal[q]] = q;
+    // first group that needs a chunk delivered, were every halo entry read through the ring
+    std::vector<int> first_need((size_t)nch + 1, ng), wmark((size_t)ng, 0);
+    for (int g = 0, run = 0; g < ng; ++g) {
+        for (int q = gfirst[g]; q < gfirst[g + 1]; ++q) {
+            const int i = C.row(rows[q]), t = C.ipos[i];
+            for (int k = C.prp[t]; k < C.prp[t + 1]; ++k) {
+                const int j = C.pci[k];
+                if (j != i && C.ord(j) < p0) run = std::max(run, S.hpos[j] / 32 + 1);
+            }
+        }
+        for (int c = (g ? wmark[g - 1] : 0); c < run; ++c) first_need[c] = g;
+        wmark[g] = run;
+    }
+    // the last ring read of each own value and each halo value
+    std::vector<int> own_last((size_t)nr, -1), halo_last((size_t)nh, -1);
+    std::deque<int> live;                    // groups whose records are in the ring, oldest first
+    std::vector<int> roff((size_t)ng), rsize((size_t)ng);
+    int ring = 0;
+    std::vector<Entry> ent;
+    std::vector<int> of_row;                 // entries of the group's rows: [ptr[r], ptr[r + 1])
+    std::vector<unsigned char> stage_of;     // 0 columns, 1 and 2 tails
+    std::vector<int> far_of;                 // row of a far entry, -1
+    std::vector<int> need_of;
+    std::vector<int> code_of;
+    int kt[3];
+    for (int g = 0; g < ng; ++g) {
+        const int q0 = gfirst[g], c = gfirst[g + 1] - q0;
+        ent.clear();
+        of_row.assign(1, 0);
+        for (int r = 0; r < c; ++r) {
+            const int i = C.row(rows[q0 + r]), t = C.ipos[i];
+            for (int k = C.prp[t]; k < C.prp[t + 1]; ++k)
+                if (C.pci[k] != i) ent.push_back({C.level[C.pci[k]], C.pci[k], k});
+            // by age; by lanes the entries stay in column order
+            if (!C.lanes)
+                std::sort(ent.begin() + of_row[r], ent.end(), [&](const Entry &a, const Entry &b) {
+                    return a.lev != b.lev ? a.lev < b.lev : C.ord(a.j) < C.ord(b.j);
+                });
+            of_row.push_back((int)ent.size());
+        }
+        stage_of.assign(ent.size(), 0);
+        code_of.assign(ent.size(), 0);
+        need_of.assign(ent.size(), 0);
+        far_of.assign(ent.size(), -1);
+        int own_need[3] = {-1, -1, -1}, halo_need[3] = {0, 0, 0};
+        int K0 = 0;
+        bool any_far = false;
+        kt[1] = kt[2] = 0;
+        const int lev = C.level[C.row(rows[q0])];
+        for (int r = 0; r < c; ++r) {
+            int k0 = 0, kr[3] = {0, 0, 0};
+            for (int e = of_row[r]; e < of_row[r + 1]; ++e) {
+                const int j = ent[e].j, d = lev - ent[e].lev;
+                const bool own = C.ord(j) >= p0;
+                bool far;
+                int need = 0;
+                if (own) {
+                    const int q = pos[C.ord(j) - p0];
+                    far = q + L.S_own < nr && g >= grp[q + L.S_own];
+                    code_of[e] = q % L.S_own;
+                    need = grp[q];
+                    if (!far) own_last[q] = g;
+                } else {
+                    const int q = S.hpos[j];
+                    const long long over = (long long)q + L.S_halo;
+                    far = over < nh && g >= first_need[over / 32];
+                    code_of[e] = L.S_own + q % L.S_halo;
+                    need = q + 1;
+                    if (!far) halo_last[q] = g;
+                }
+                int s = !C.lanes && d <= TS_TAILS ? TS_TAILS + 1 - d : 0;
+                if (s && kr[s] >= TS_TAIL) s = 0;
+                if (far) {
+                    if (s) {
+                        O.why = "a newest dependency left its ring";
+                        break;
+                    }
+                    code_of[e] = TS_FAR;
+                    far_of[e] = j;
+                    any_far = true;
+                    ++O.nfar;
+                    ++k0;
+                    continue;
+                }
+                stage_of[e] = (unsigned char)s;
+                need_of[e] = need;
+                if (s == 0) {
+                    ++k0;
+                    continue;
+                }
+                ++kr[s];
+                if (own) own_need[s] = std::max(own_need[s], need);
+                else halo_need[s] = std::max(halo_need[s], need);
+            }
+            K0 = std::max(K0, k0);
+            for (int s = 1; s <= TS_TAILS; ++s) kt[s] = std::max(kt[s], kr[s]);
+        }
+        if (O.why) break;
+        // the group overwrites the own-ring slots of its rows: their last readers first
+        for (int q = q0; q < q0 + c; ++q)
+            if (q >= L.S_own) own_need[TS_TAILS] = std::max(own_need[TS_TAILS], own_last[q - L.S_own]);
+        // lanes a row in the columns: two where they fit (half the columns for one more addition)
+        int lg = 0;
+        if (C.lanes) lg = C.lanes == 4 ? 2 : 3;
+        else if (c <= 16 && K0 > 2) lg = 1;
+        const int G = 1 << lg, blk = C.lanes ? 1 : 4;
+        const int D0 = (K0 + G - 1) / G, KT = kt[1] + kt[2], nb = (D0 + blk - 1) / blk;
+        if (nb > 65535) {
+            O.why = "a row with too many entries";
+            break;
+        }
+        const TileRec R = tile_rec(c, nb, blk, any_far, KT, elem);
+        if (R.size > L.B_rec / 2) {
+            O.why = "a group's record does not fit the staging ring";
+            break;
+        }
+        // place in the ring: the groups whose bytes it takes must be done
+        int need = g - TS_NM;
+        auto drop = [&]() {
+            need = std::max(need, live.front());
+            live.pop_front();
+        };
+        if (ring + R.size > L.B_rec) {
+            // what the previous lap left behind this lap's end is older than what it left at the start
+            while (!live.empty() && roff[live.front()] >= ring) drop();
+            ring = 0;
+        }
+        while (!live.empty() && roff[live.front()] < ring + R.size && roff[live.front()] + rsize[live.front()] > ring)
+            drop();
+        roff[g] = ring;
+        rsize[g] = R.size;
+        live.push_back(g);
+        const size_t base = O.rec.size();
+        O.groups.push_back((int)(base / 16));
+        O.groups.push_back(R.size / 16);
+        O.groups.push_back(ring / 16);
+        O.groups.push_back(std::max(need, -1));
+        ring += R.size;
+        O.rec.resize(base + (size_t)R.size, 0);
+        unsigned char *rec = O.rec.data() + base;
+        int *hd = (int *)rec;
+        hd[0] = c | lg << 8 | kt[1] << 16 | kt[2] << 20;
+        hd[1] = nb | (any_far ? 1 << 16 : 0);
+        hd[2] = q0 % L.S_own;
+        hd[3] = D0 - blk * (nb - 1);
+        for (int s = 1; s <= TS_TAILS; ++s) {
+            hd[2 + 2 * s] = own_need[s];
+            hd[3 + 2 * s] = halo_need[s];
+        }
+        hd[12] = R.o_old / 16 | R.o_tail / 16 << 16;
+        hd[13] = R.o_cold / 16 | R.o_ctail / 16 << 16;
+        hd[14] = R.o_cfar / 16;
+        hd[15] = R.o_row / 16 | R.o_lv / 16 << 16;
+        int *need_b = (int *)(rec + R.o_need);
+        for (int q = 0; q < nb; ++q) need_b[2 * q] = -1;
+        int *rid = (int *)(rec + R.o_row), *cfar = (int *)(rec + R.o_cfar);
+        unsigned short *cold = (unsigned short *)(rec + R.o_cold), *ctail = (unsigned short *)(rec + R.o_ctail);
+        const unsigned short pad = (unsigned short)(L.S_own + L.S_halo);
+        for (int q = 0; q < 32 * blk * nb; ++q) cold[q] = pad;
+        for (int q = 0; q < 32 * KT; ++q) ctail[q] = pad;
+        const int e_old = (int)((base + R.o_old) / elem), e_tail = (int)((base + R.o_tail) / elem),
+                  e_lv = (int)((base + R.o_lv) / elem);
+        for (int r = 0; r < c; ++r) {
+            const int i = C.row(rows[q0 + r]), t = C.ipos[i];
+            rid[r] = i;
+            C.dlv[t] = e_lv + r;
+            for (int k = C.prp[t]; k < C.prp[t + 1]; ++k)
+                if (C.pci[k] == i) C.dval[k] = -1;
+            // by age right-aligned: a short row's entries are as recent as the others' last ones
+            int k0 = C.lanes ? 0 : 4 * nb * G, kr[3] = {0, 0, kt[1]};
+            for (int e = of_row[r]; e < of_row[r + 1] && !C.lanes; ++e) k0 -= stage_of[e] == 0;
+            for (int e = of_row[r]; e < of_row[r + 1]; ++e) {
+                if (stage_of[e] == 0) {
+                    const int q = k0 / G, lane = r * G + k0 % G, b = q / blk;
+                    if (far_of[e] < 0) {
+                        int &m = need_b[2 * b + (C.ord(ent[e].j) < p0)];
+                        m = std::max(m, need_of[e]);
+                    } else {
+                        cfar[32 * blk * b + blk * lane + q % blk] = far_of[e];
+                    }
+                    cold[32 * blk * b + blk * lane + q % blk] = (unsigned short)code_of[e];
+                    C.dval[ent[e].k] = e_old + 32 * blk * b + ts_col(q % blk, lane, blk, elem);
+                    ++k0;
+                } else {
+                    const int at = kr[stage_of[e]]++ * 32 + r;
+                    ctail[at] = (unsigned short)code_of[e];
+                    C.dval[ent[e].k] = e_tail + at;
+                }
+            }
+        }
+    }
+    // halo values: rows, and the group after whose end the slots' previous values are dead
+    O.halo.assign((size_t)nch * 32, -1);
+    O.rel.assign((size_t)nch, -1);
+    for (int q = 0; q < nh; ++q) {
+        O.halo[q] = hal[q];
+        if (q >= L.S_halo) O.rel[q / 32] = std::max(O.rel[q / 32], halo_last[q - L.S_halo]);
+    }
+    for (int h : hal) S.hpos[h] = -1;
+}
+
+int plan_threads() {
+    if (const char *e = std::getenv("SSG_PLAN_THREADS")) {
+        const int v = std::atoi(e);
+        if (v >= 1 && v <= 64) return v;
+    }
+    const unsigned hc = std::thread::hardware_concurrency();
+    return (int)std::max(1u, std::min(16u, hc / 2));
+}
+
+}  // namespace
+
+TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level,
+                            bool lower, int elem, int lanes, int T, const TileLayout *lay) {
+    TilePlanHost P;
+    auto fail = [&](const char *why) {
+        P.ok = false;
+        P.why = why;
+        return P;
+    };
+    if (n <= 0) return fail("no rows");
+    if (T <= 0) T = tile_count(n);
+    T = std::min(T, n);
+    P.T = T;
+    P.lay = lay ? *lay : tile_layout(elem);
+    P.dval.assign((size_t)prp[n], -1);
+    P.dlv.assign((size_t)n, 0);
+    const Ctx C{n, elem, lanes, prp, pci, ipos, level, lower, P.lay, P.dval.data(), P.dlv.data()};
+    std::vector<TileOut> out((size_t)T);
+    auto first = [&](int t) { return (int)((long long)n * t / T); };
+    {
+        const int nt = std::max(1, std::min(plan_threads(), T));
+        std::atomic<int> next{0};
+        std::vector<std::exception_ptr> errs((size_t)nt);
+        auto work = [&](int q) {
+            try {
+                Scratch S(n);
+                for (int t; (t = next.fetch_add(1)) < T;) plan_tile(C, first(t), first(t + 1), S, out[t]);
+            } catch (...) {
+                errs[q] = std::current_exception();
+            }
+        };
+        std::vector<std::thread> pool;
+        for (int q = 1; q < nt; ++q) {
+            try {
+                pool.emplace_back(work, q);
+            } catch (...) {
+                break;  // fewer threads: the others take its tiles
+            }
+        }
+        work(0);
+        for (auto &t : pool) t.join();
+        for (auto &e : errs)
+            if (e) std::rethrow_exception(e);
+    }
+    long long off = 0, g0 = 0, c0 = 0;
+    P.tiles.resize((size_t)T * 4);
+    P.rec.resize((size_t)T);
+    P.rec_off.resize((size_t)T + 1);
+    for (int t = 0; t < T; ++t) {
+        if (out[t].why) return fail(out[t].why);
+        P.rec_off[t] = off;
+        P.tiles[4 * t] = (int)g0;
+        P.tiles[4 * t + 1] = (int)out[t].groups.size() / 4;
+        P.tiles[4 * t + 2] = (int)c0;
+        P.tiles[4 * t + 3] = (int)out[t].rel.size();
+        g0 += (long long)out[t].groups.size() / 4;
+        c0 += (long long)out[t].rel.size();
+        off += (long long)out[t].rec.size();
+        P.nfar += out[t].nfar;
+    }
+    P.rec_off[T] = off;
+    P.rec_bytes = off;
+    if (off / elem >= (1ll << 31) || g0 >= (1ll << 29) || c0 >= (1ll << 26)) return fail("records too large");
+    P.groups.resize((size_t)g0 * 4);
+    P.halo.resize((size_t)c0 * 32);
+    P.rel.resize((size_t)c0);
+    for (int t = 0; t < T; ++t) {
+        const int r16 = (int)(P.rec_off[t] / 16), rel_e = (int)(P.rec_off[t] / elem);
+        TileOut &o = out[t];
+        for (size_t q = 0; q < o.groups.size(); q += 4) o.groups[q] += r16;
+        std::copy(o.groups.begin(), o.groups.end(), P.groups.begin() + (size_t)P.tiles[4 * t] * 4);
+        std::copy(o.halo.begin(), o.halo.end(), P.halo.begin() + (size_t)P.tiles[4 * t + 2] * 32);
+        std::copy(o.rel.begin(), o.rel.end(), P.rel.begin() + (size_t)P.tiles[4 * t + 2]);
+        for (int p = first(t); p < first(t + 1); ++p) {
+            const int i = lower ? p : n - 1 - p, q = ipos[i];
+            P.dlv[q] += rel_e;
+            for (int k = prp[q]; k < prp[q + 1]; ++k)
+                if (P.dval[k] >= 0) P.dval[k] += rel_e;
+        }
+        P.rec[t] = std::move(o.rec);
+    }
+    P.ok = true;
+    return P;
+}
+
+}  // namespace ssg
