@@ -236,23 +236,29 @@ __global__ void __launch_bounds__(256) k_ic_factor(int n, const int *perm, const
 // subtracts its contribution L_ik L_jk D_k (when column k also appears in
 // row j) -- the same terms, subtracted in the same order, as the reference's
 // loop over kk, so with FMA contraction off (this file is compiled with
-// -fmad=false) the real factor is bit-identical to the reference's. Before a
-// lane waits for row j (its entry's column), it stages row j's columns (the
-// row's start in the level-ordered arrays comes from a per-entry table built
-// once per pattern) and finds where row j holds each earlier column of row i;
-// once row j's done flag is seen, only its pivot and those values are loaded.
+// -fmad=false) the real factor is bit-identical to the reference's.
+//
+// What bounds it: the dependency levels, each one row's work after the newest row it reads. k_ic_factor_flow keeps that
+// short: the output starts as sentinels, so a row's values are their own ready flags (no fence, no flag store, no flag
+// poll between a row and its readers); what needs the pattern alone (the columns of row j = c, and which step uses each)
+// is found before the wait; after it a lane loads all the values it needs at once; and row i's own reads of A replace the
+// pass that used to copy the lower triangle first.
+// Measured (GB300, ms a factor, with done flags and a wait loop a lane -> now): real 10^3 1.96 -> 0.60, 20^3 4.57 -> 1.40,
+// 41^3 10.1 -> 3.13, 80^3 25.2 -> 8.4; complex 12^3 5.6 -> 1.97, 33^3 16.8 -> 6.6, 60^3 34.6 -> 16.6. At 80^3 a level of the
+// chain is now 5.9 us, of which the update loop about 2.4 (15 steps of 314 cycles), reading the newest rows 1.5 to 2 and
+// the division 0.6; its FP64 instructions alone would take 5.4 ms on all SMs.
 constexpr int FF_MAXROW = 32;
-int factor_blocks_per_sm = 4;  // rows in flight: enough for a level, few enough not to congest L2
+constexpr int factor_blocks_per_sm = 4;  // k_ic_factor_nat
+constexpr int factor_rows_per_sm = 16;   // rows in flight: enough for a level, few enough not to congest L2
 template <typename T>
 __host__ __device__ constexpr int ff_warps() { return sizeof(T) == 8 ? 3 : 2; }  // static shared memory below 48 KB
 
-// NAT: rows in natural order (perm is the identity, a row's dependencies start
-// at prp[c]); dep and perm are then not read.
-template <typename T, bool NAT = false>
-__global__ void __launch_bounds__(ff_warps<T>() * 32) k_ic_factor_fast(int n, const int *perm, const int *prp,
-                                                                       const int *pci, const int2 *dep, T *lval,
-                                                                       T *D, int *done, double alpha, int *ticket,
-                                                                       int *err, int backoff_ns, const int *sub) {
+// The factor without allocation: rows in natural order (a row's dependencies start at prp[c]), in place, with done flags.
+// Before a lane waits for row j it stages row j's columns and finds where row j holds each earlier column of row i.
+template <typename T>
+__global__ void __launch_bounds__(ff_warps<T>() * 32) k_ic_factor_nat(int n, const int *prp, const int *pci, T *lval,
+                                                                      T *D, int *done, double alpha, int *ticket,
+                                                                      int *err) {
     constexpr int FF_WARPS = ff_warps<T>();
     __shared__ int s_c[FF_WARPS][FF_MAXROW][FF_MAXROW - 1];            // columns of row j
     __shared__ unsigned char s_p[FF_WARPS][FF_MAXROW][FF_MAXROW - 1];  // step kk: position of c_kk in row j
@@ -263,8 +269,7 @@ __global__ void __launch_bounds__(ff_warps<T>() * 32) k_ic_factor_fast(int n, co
         if (lane == 0) t = atomicAdd(ticket, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= n) return;
-        if (!NAT && sub) t = sub[t];
-        const int i = NAT ? t : perm[t];
+        const int i = t;
         const int a = prp[t], m = prp[t + 1] - a;
         const bool have = lane < m;
         const int c = have ? pci[a + lane] : INT_MAX;
@@ -274,7 +279,7 @@ __global__ void __launch_bounds__(ff_warps<T>() * 32) k_ic_factor_fast(int n, co
         // ascend strictly (the merge below walks both rows in column order)
         const int prev_c = __shfl_up_sync(0xffffffffu, c, 1);
         const bool bad_col =
-            NAT && __any_sync(0xffffffffu, have && ((lane < m - 1 && (c < 0 || c >= i)) || (lane > 0 && prev_c >= c)));
+            __any_sync(0xffffffffu, have && ((lane < m - 1 && (c < 0 || c >= i)) || (lane > 0 && prev_c >= c)));
         if (m < 1 || m > FF_MAXROW || last_c != i || bad_col) {
             // no diagonal last (src/SprsPreconditioner.cpp:88-94), a bad caller pattern, or too long
             if (lane == 0) {
@@ -295,7 +300,7 @@ __global__ void __launch_bounds__(ff_warps<T>() * 32) k_ic_factor_fast(int n, co
         int mj = 0;
         unsigned hits = 0u;  // bit kk: row j holds column c_kk
         if (off) {
-            dj = NAT ? make_int2(prp[c], prp[c + 1] - prp[c]) : dep[a + lane];
+            dj = make_int2(prp[c], prp[c + 1] - prp[c]);
             mj = min(dj.y - 1, FF_MAXROW - 1);
 #pragma unroll
             for (int l = 0; l < FF_MAXROW - 1; ++l)
@@ -321,7 +326,6 @@ __global__ void __launch_bounds__(ff_warps<T>() * 32) k_ic_factor_fast(int n, co
                 const unsigned long long start = gtimer();
                 int polls = 0;
                 while (*f == 0) {
-                    if (backoff_ns) __nanosleep(backoff_ns);
                     if ((++polls & 15) == 0) {
                         if (*(volatile int *)err) break;
                         if (gtimer() - start > spin_limit_ns(err)) {
@@ -360,6 +364,138 @@ __global__ void __launch_bounds__(ff_warps<T>() * 32) k_ic_factor_fast(int n, co
     }
 }
 
+// one value of the factor under construction; false while its row is not done
+__device__ __forceinline__ bool take(const double *p, double &v) {
+    v = ld_vol(p);
+    return !is_sent(v);
+}
+__device__ __forceinline__ bool take(const cplx *p, cplx &v) {
+    v.x = ld_vol(&p->x);
+    v.y = ld_vol(&p->y);
+    return !is_sent(v.x) && !is_sent(v.y);
+}
+__device__ __forceinline__ void give(double *p, double v) { st_vol(p, unsent(v)); }
+__device__ __forceinline__ void give(cplx *p, cplx v) {
+    st_vol(&p->x, unsent(v.x));
+    st_vol(&p->y, unsent(v.y));
+}
+
+// MAXL: entries of a row at most, the diagonal included. lval and D hold sentinels at launch; aval[psrc[k]] is entry k of A.
+template <typename T, int MAXL>
+__host__ __device__ constexpr int fl_warps() { return sizeof(T) * MAXL > 320 ? 2 : 4; }  // static shared memory below 48 KB
+template <typename T, int MAXL>
+__global__ void __launch_bounds__(fl_warps<T, MAXL>() * 32)
+    k_ic_factor_flow(int n, const int *__restrict__ perm, const int *__restrict__ prp, const int *__restrict__ pci,
+                     const int2 *__restrict__ dep, const int *__restrict__ psrc, const T *__restrict__ aval, T *lval, T *D,
+                     double alpha, int *ticket, int *err, int backoff_ns, const int *__restrict__ sub) {
+    __shared__ T s_v[fl_warps<T, MAXL>()][MAXL - 1][32];  // step kk: L_jk of the lane's row j
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(ticket, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= n) return;
+        if (sub) t = sub[t];
+        const int i = perm[t];
+        const int a = prp[t], m = prp[t + 1] - a;
+        const bool have = lane < m;
+        const int c = have ? pci[a + lane] : INT_MAX;
+        T v = have ? aval[psrc[a + lane]] : Sc<T>::zero();
+        const int last_c = __shfl_sync(0xffffffffu, c, (m - 1) & 31);
+        if (m < 1 || m > MAXL || last_c != i) {
+            // no diagonal last (src/SprsPreconditioner.cpp:88-94)
+            if (lane == 0) atomicExch(err, m > MAXL ? ERR_ROW_TOO_LONG : ERR_NO_DIAG);
+            if (have) give(lval + a + lane, Sc<T>::zero());
+            if (lane == 0) give(D + i, Sc<T>::one());
+            continue;
+        }
+        const bool off = lane < m - 1;  // off-diagonal entry (column c < i): row j = c
+        // Which step uses each entry l of row j (its diagonal, the last, aside): the place of its column among row i's,
+        // by binary search over the lanes; -1 none before this lane's.
+        int2 dj = make_int2(0, 1);
+        if (off) dj = dep[a + lane];
+        int step[MAXL - 1];
+#pragma unroll
+        for (int l = 0; l < MAXL - 1; ++l) step[l] = l < dj.y - 1 ? __ldg(pci + dj.x + l) : INT_MAX;
+        unsigned hits = 0u;  // bit kk: row j holds column c_kk
+#pragma unroll
+        for (int l = 0; l < MAXL - 1; ++l) {
+            const int x = step[l];
+            step[l] = -1;
+            if (!__any_sync(0xffffffffu, x != INT_MAX)) continue;
+            int kk = 0;
+#pragma unroll
+            for (int h = 16; h >= 1; h >>= 1)
+                if (__shfl_sync(0xffffffffu, c, kk + h - 1) < x) kk += h;
+            const int ck = __shfl_sync(0xffffffffu, c, kk & 31);
+            if (ck == x && kk < lane) {
+                step[l] = kk;
+                hits |= 1u << kk;
+            }
+        }
+        // Every wait below is one loop of the whole warp. Lanes that leave a loop of their own stay apart afterwards, and
+        // each part of a warp takes the FP64 pipe for its own 64 cycles an instruction: with a loop a lane the update
+        // below ran in about seven parts, 1,400 cycles a step instead of 300.
+        auto wait_all = [&](bool have, const T *p, T &x) {
+            if (__all_sync(0xffffffffu, have)) return;
+            const unsigned long long start = gtimer();
+            int polls = 0;
+            do {
+                if (backoff_ns) __nanosleep(backoff_ns);
+                if (!have) have = take(p, x);
+                if ((++polls & 15) == 0) {
+                    const bool late = gtimer() - start > spin_limit_ns(err);
+                    if (__any_sync(0xffffffffu, late || *(volatile int *)err != 0)) {
+                        if (late) atomicExch(err, ERR_TIMEOUT);
+                        break;
+                    }
+                }
+            } while (!__all_sync(0xffffffffu, have));
+            __syncwarp();
+        };
+        // row j is done, or nearly, when its diagonal is; each value still tells for itself
+        T x;
+        wait_all(!off, lval + dj.x + max(dj.y - 1, 0), x);
+        T val[MAXL - 1];
+        unsigned miss = 0u;
+#pragma unroll
+        for (int l = 0; l < MAXL - 1; ++l) {
+            val[l] = Sc<T>::zero();
+            if (off && step[l] >= 0 && !take(lval + dj.x + l, val[l])) miss |= 1u << l;
+        }
+        if (__any_sync(0xffffffffu, miss != 0u)) {
+#pragma unroll
+            for (int l = 0; l < MAXL - 1; ++l) wait_all(!((miss >> l) & 1u), lval + dj.x + l, val[l]);
+        }
+#pragma unroll
+        for (int l = 0; l < MAXL - 1; ++l)
+            if (off && step[l] >= 0) s_v[w][step[l]][lane] = val[l];
+        T dk = Sc<T>::zero();
+        wait_all(!off, D + c, dk);  // the pivot's reciprocal comes a division later
+        __syncwarp();
+        // diagonal lane starts from alpha * a_ii (src/SprsPreconditioner.cpp:95)
+        const bool diag = lane == m - 1;
+        if (diag) {
+            v = v * Sc<T>::from(alpha);
+            hits = 0xffffffffu;
+        }
+#pragma unroll 1
+        for (int kk = 0; kk < m - 1; ++kk) {
+            const T Lk = Sc<T>::shfl(v, kk);  // final L_ik
+            const T Dk = Sc<T>::shfl(dk, kk);
+            // an off-diagonal lane subtracts L_ik L_jk D_k when row j holds column k; the
+            // diagonal lane L_ik L_ik D_k: one update for both
+            if ((hits >> kk) & 1u) {
+                const T o = diag ? Lk : s_v[w][kk][lane];
+                v = v - (Lk * o) * Dk;
+            }
+        }
+        if (have) give(lval + a + lane, v);
+        if (diag) give(D + i, (Sc<T>::absv(v) < 1.0e-12) ? Sc<T>::from(1.0 / DBL_EPSILON) : Sc<T>::one() / v);
+        __syncwarp();
+    }
+}
+
 __global__ void k_dep_starts(int nnz, const int *pci, const int *ipos, const int *prp, int2 *dep) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nnz) return;
@@ -389,25 +525,32 @@ void factor_plan(const Tri &L, DBuf &dep, int &max_row, cudaStream_t s) {
 }
 
 template <typename T>
-void ic_factor(const Tri &L, T *lval, T *D, double alpha, int *d_err, int *d_ticket, cudaStream_t s,
+void ic_factor(const Tri &L, const T *aval, T *lval, T *D, double alpha, int *d_err, int *d_ticket, cudaStream_t s,
                const int2 *dep, int max_row, int *done, int backoff_ns, const int *sub, int nsub) {
     if (L.n == 0) return;
     const int cnt = sub ? nsub : L.n;  // rows to factor (sub: their level-ordered positions, ascending)
     if (cnt == 0) return;
-    SSG_CUDA(cudaMemsetAsync(done, 0, sizeof(int) * (size_t)L.n, s));
     SSG_CUDA(cudaMemsetAsync(d_ticket, 0, sizeof(int), s));
     int dev = 0, sms = 0;
     SSG_CUDA(cudaGetDevice(&dev));
     SSG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (dep && max_row <= FF_MAXROW) {
-        constexpr int W = ff_warps<T>();
+        // all bits set is the sentinel
+        SSG_CUDA(cudaMemsetAsync(lval, 0xFF, sizeof(T) * (size_t)L.nnz, s));
+        SSG_CUDA(cudaMemsetAsync(D, 0xFF, sizeof(T) * (size_t)L.n, s));
         // wide levels (batches of many systems) keep more rows in flight
         const double width = L.nlev > 0 ? (double)cnt / L.nlev : (double)cnt;
-        const int per_sm = width >= 8192.0 ? 6 : factor_blocks_per_sm;
-        const int blocks = min(div_up(cnt, W), sms * per_sm);
-        k_ic_factor_fast<T><<<blocks, W * 32, 0, s>>>(cnt, L.perm.as<int>(), L.prp.as<int>(), L.pci.as<int>(), dep,
-                                                      lval, D, done, alpha, d_ticket, d_err, backoff_ns, sub);
+        const int rows_per_sm = width >= 8192.0 ? 24 : factor_rows_per_sm;
+        auto launch = [&](auto kern, int W) {
+            kern<<<min(div_up(cnt, W), sms * (rows_per_sm / W)), W * 32, 0, s>>>(
+                cnt, L.perm.as<int>(), L.prp.as<int>(), L.pci.as<int>(), dep, L.psrc.as<int>(), aval, lval, D, alpha,
+                d_ticket, d_err, backoff_ns, sub);
+        };
+        if (max_row <= 20) launch(k_ic_factor_flow<T, 20>, fl_warps<T, 20>());
+        else launch(k_ic_factor_flow<T, FF_MAXROW>, fl_warps<T, FF_MAXROW>());
     } else {
+        gather_values<T>(L.psrc.as<int>(), aval, lval, L.nnz, s);
+        SSG_CUDA(cudaMemsetAsync(done, 0, sizeof(int) * (size_t)L.n, s));
         const int warps = min(cnt, sms * 32);
         k_ic_factor<T><<<div_up(warps * 32, 256), 256, 0, s>>>(cnt, L.perm.as<int>(), L.ipos.as<int>(),
                                                                L.prp.as<int>(), L.pci.as<int>(), lval, D, done,
@@ -526,7 +669,7 @@ void all_pivots_positive(int n, const T *D, int *d_flag, cudaStream_t s) {
 }
 
 #define SSG_INST(T)                                                                                      \
-    template void ic_factor<T>(const Tri &, T *, T *, double, int *, int *, cudaStream_t, const int2 *, int,  \
+    template void ic_factor<T>(const Tri &, const T *, T *, T *, double, int *, int *, cudaStream_t, const int2 *, int,  \
                                int *, int, const int *, int);                                                \
     template void copy_replica_rows<T>(const Tri &, const int *, T *, T *, cudaStream_t);                     \
     template void diag_scaling<T>(int, const int *, const int *, const T *, const T *, T *, T *,        \
@@ -568,8 +711,7 @@ static cudaError_t noalloc_launch(int n, const int *lrp, const int *lci, void *l
                                   int *scr, int sms, cudaStream_t s) {
     constexpr int W = ff_warps<T>();
     const int blocks = min(div_up(n, W), sms * factor_blocks_per_sm);
-    k_ic_factor_fast<T, true><<<blocks, W * 32, 0, s>>>(n, nullptr, lrp, lci, nullptr, (T *)lval, (T *)D,
-                                                        scr + NA_HEAD, alpha, scr, scr + 1, 0, nullptr);
+    k_ic_factor_nat<T><<<blocks, W * 32, 0, s>>>(n, lrp, lci, (T *)lval, (T *)D, scr + NA_HEAD, alpha, scr, scr + 1);
     return cudaGetLastError();
 }
 

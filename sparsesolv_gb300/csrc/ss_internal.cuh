@@ -137,9 +137,9 @@ void gather_values(const int *src, const T *in, T *out, int count, cudaStream_t 
 // ss_factor.cu
 // per entry of L: (start, length) of its dependency row in level order; longest row
 void factor_plan(const Tri &L, DBuf &dep, int &max_row, cudaStream_t s);
-// asynchronous; done[n] is scratch the caller owns
+// asynchronous; aval[L.psrc[k]] is entry k; done[n] is scratch the caller owns
 template <typename T>
-void ic_factor(const Tri &L, T *lval, T *D, double alpha, int *d_err, int *d_ticket, cudaStream_t s,
+void ic_factor(const Tri &L, const T *aval, T *lval, T *D, double alpha, int *d_err, int *d_ticket, cudaStream_t s,
                const int2 *dep, int max_row, int *done, int backoff_ns, const int *sub = nullptr, int nsub = 0);
 // copy the factor rows of rows with a source row (rep_src[i] >= 0) from that row
 template <typename T>

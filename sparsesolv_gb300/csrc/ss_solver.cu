@@ -269,9 +269,8 @@ void Handle::ensure_factor(double alpha, bool scaled) {
         fac_sub_valid = true;
     }
     auto factor_once = [&](double a) {
-        gather_values<T>(Lf.psrc.as<int>(), aval, Lval.as<T>(), nnzL, stream);
         timed(PC_FACTOR, 2.0 * (4.0 + sizeof(T)) * nnzL + (double)sizeof(T) * n, [&] {
-            ic_factor<T>(Lf, Lval.as<T>(), Dvec.as<T>(), a, err(), ticket() + 2, stream, dep.as<int2>(), max_row,
+            ic_factor<T>(Lf, aval, Lval.as<T>(), Dvec.as<T>(), a, err(), ticket() + 2, stream, dep.as<int2>(), max_row,
                          done_buf.as<int>(), fac_backoff_ns, rep_on ? fac_sub.as<int>() : nullptr, fac_sub_n);
             if (rep_on) copy_replica_rows<T>(Lf, rep_src.as<int>(), Lval.as<T>(), Dvec.as<T>(), stream);
         });

@@ -219,15 +219,17 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
         auto record = [&](int g) -> const unsigned char * {
             const unsigned bar = full + 8u * (g % TS_NM);
             const unsigned par = (unsigned)((g / TS_NM) & 1);
-            if (!tl_mbar_test(bar, par)) {
+            // one loop of the whole warp, as everywhere here: lanes that leave loops of their own stay apart afterwards, and
+            // each part of a warp takes the FP64 pipe for itself
+            bad = __any_sync(0xffffffffu, bad);
+            if (!bad && !__all_sync(0xffffffffu, tl_mbar_test(bar, par))) {
                 Bound b(a.err, lim);
-                while (!tl_mbar_test(bar, par))
-                    if (b.spent(255)) {
+                while (!__all_sync(0xffffffffu, tl_mbar_test(bar, par)))
+                    if (__any_sync(0xffffffffu, b.spent(255))) {
                         bad = true;
                         break;
                     }
             }
-            bad = __any_sync(0xffffffffu, bad);
             return bad ? nullptr : tl_smem + L.o_rec + 16 * place[g % TS_NM];
         };
 
@@ -245,16 +247,19 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                 const T *v = (const T *)(rec + 16 * (of.x & 0xffff));
                 // a column's value: from the rings, or from memory where its slot is reused too early
                 auto value = [&](int code, const int *far_row) -> T {
-                    if (code != TS_FAR) return X[code];
                     T x = Sc<T>::zero();
-                    if (!tl_take(out + *far_row, x)) {
-                        Bound b(a.err, lim);
-                        while (!tl_take(out + *far_row, x))
-                            if (b.spent(63)) {
-                                bad = true;
-                                break;
-                            }
-                    }
+                    bool have = code != TS_FAR;
+                    if (have) x = X[code];
+                    if (__all_sync(0xffffffffu, have)) return x;
+                    const T *p = out + (have ? 0 : *far_row);
+                    Bound b(a.err, lim);
+                    do {
+                        if (!have) have = tl_take(p, x);
+                        if (__any_sync(0xffffffffu, b.spent(63))) {
+                            bad = true;
+                            break;
+                        }
+                    } while (!__all_sync(0xffffffffu, have));
                     return x;
                 };
                 T res = Sc<T>::zero(), u0 = res;
@@ -283,7 +288,6 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                         wait_for(w.x, w.y);
                         acc = madd(acc, vv, cfar ? value(cc, cfar + 32 * k + lane) : X[cc]);
                     }
-                    if (cfar) __syncwarp();
 #pragma unroll
                     for (int m = LANES / 2; m >= 1; m >>= 1) acc = acc + Sc<T>::shfl_xor(acc, m);
                     if (MODE == SW_BWD_IC) res = madd(u0, lv, acc);
@@ -321,7 +325,6 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                         } else {
                             const int *f = cfar + 128 * k + 4 * lane;
                             x0 = value(cc.x, f), x1 = value(cc.y, f + 1), x2 = value(cc.z, f + 2), x3 = value(cc.w, f + 3);
-                            __syncwarp();
                         }
                         // jumps, not predicates, past the first block's empty columns: a multiply-add costs the FP64
                         // latency whether or not it runs
