@@ -1340,12 +1340,12 @@ void Batch::precond32(const Ti *r, Ti *z, const KState *stp) {
     SSG_CUDA(cudaMemsetAsync(y, 0xFF, v * (size_t)n, s));
     h.timed(PC_FWD, fb, [&] {
         sweep_st<Ti>(h.Lf, L32.as<Ti>(), SW_FWD_DIV, r, nullptr, nullptr, y, nullptr, h.ticket(), h.err(), stp, s,
-                     h.swcfg, h.use_inv_diag ? invL32.as<Ti>() : nullptr);
+                     h.free_cfg(h.Lf), h.use_inv_diag ? invL32.as<Ti>() : nullptr);
     });
     SSG_CUDA(cudaMemsetAsync(z, 0xFF, v * (size_t)n, s));
     h.timed(PC_BWD, fb + v * n, [&] {
         sweep_st<Ti>(h.Ltb, Lt32.as<Ti>(), SW_BWD_IC, nullptr, y, D32.as<Ti>(), z, nullptr, h.ticket() + 1, h.err(),
-                     stp, s, h.swcfg, (const Ti *)nullptr);
+                     stp, s, h.free_cfg(h.Ltb), (const Ti *)nullptr);
     });
 }
 
@@ -1528,7 +1528,7 @@ int solve_batched(Handle &h, Batch *&mb, uint64_t &mver, uint64_t &mpat, int pre
     mb->h.swcfg.cta_per_sm = h.swcfg.cta_per_sm;
     mb->h.sweep_mode = h.sweep_mode;
     // a handle's own batch (mixed precision, several right-hand sides) serves one matrix:
-    // its automatic mode may take the push sweep, as the handle's single solves do
+    // its automatic mode may take the sweeps of the handle's single solves
     mb->h.push_auto = true;
     if (mb->h.spin_limit_us != h.spin_limit_us) mb->h.set_spin_limit(h.spin_limit_us);
     AllocStream as(mb->h.stream);  // the batch's buffers are ordered on its own stream

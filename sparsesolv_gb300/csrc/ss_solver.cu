@@ -343,14 +343,22 @@ static double tri_bytes(const Tri &T, size_t v, int vecs) {
     return (4.0 + (double)v) * T.nnz + 4.0 * (T.n + 1) + (double)vecs * (double)v * T.n;
 }
 
-// mean rows per level above which the automatic mode keeps the sync-free sweep
-static constexpr double kAutoClusterRowsPerLevel = 4096.0;
+// mean rows per level up to which a triangle's levels are narrow: latency, not the row count, sets the pace
+static constexpr double kNarrowRowsPerLevel = 4096.0;
+static bool narrow(const Tri &t) { return (double)t.n <= kNarrowRowsPerLevel * (double)t.nlev; }
+
+// What serves where the tile sweeps do not: the sync-free sweep, in the lanes a row (and so with the bits) of the
+// one-cluster sweep it replaced there as the automatic choice. Measured at 8 lanes a row, us forward: 10^3 190 (lockstep
+// cluster 263, push 221), 20^3 438 (583, 497), 41^3 960 (1,405, 1,088), 80^3 2,094 (4,435, 2,226), complex 33^3 1,277
+// (1,497). The one-cluster and push sweeps run where SSG_TUNE_SWEEP_MODE asks for them.
+SweepCfg Handle::free_cfg(const Tri &t) const {
+    SweepCfg c = swcfg;
+    if (sweep_mode == 0 && narrow(t)) c.group = vtype == SSG_COMPLEX || !push_auto ? cl_group : 8;
+    return c;
+}
 
 bool Handle::cluster_ok(Tri &t, size_t elem, bool ic) {
-    if (sweep_mode == 1 || t.n == 0) return false;
-    // automatic: one cluster wins while the levels are narrow enough that the
-    // per-level latency, not the row count, sets the pace
-    if (sweep_mode == 0 && (double)t.n > kAutoClusterRowsPerLevel * (double)t.nlev) return false;
+    if (sweep_mode <= 1 || t.n == 0) return false;
     // the neighbour-synchronised plan (mode 3) serves IC sweeps; a triangle whose plan
     // is infeasible under it falls back to the lockstep plan
     const bool p2p = ic && sweep_mode == 3 && !(t.cl_fail & 2);
@@ -372,15 +380,9 @@ bool Handle::cluster_ok(Tri &t, size_t elem, bool ic) {
     return t.cl_ready && (ic || !t.cl_p2p);
 }
 
-// the push sweep (IC pair, with the reciprocal diagonal): forced by mode 4; the automatic
-// choice for real values wherever the one-cluster sweep would be and both push plans fit
+// the push sweep (IC pair, with the reciprocal diagonal) where mode 4 asks for it and both plans fit
 bool Handle::push_ok(size_t elem) {
-    if (!use_inv_diag || Lf.n == 0) return false;
-    if (sweep_mode != 4 && sweep_mode != 0) return false;
-    for (const Tri *t : {&Lf, &Ltb})
-        if (sweep_mode == 0 &&
-            (!push_auto || vtype == SSG_COMPLEX || (double)t->n > kAutoClusterRowsPerLevel * (double)t->nlev))
-            return false;
+    if (!use_inv_diag || Lf.n == 0 || sweep_mode != 4) return false;
     Tri *pair[2] = {&Lf, &Ltb};
     return push_plan(pair, 2, elem, stream);
 }
@@ -392,8 +394,7 @@ bool Handle::tile_ok(Tri &a, Tri &b, size_t elem) {
     if (!use_inv_diag || sweep_mode != 0 || !push_auto || a.n == 0) return false;
     const int lanes = vtype == SSG_COMPLEX ? cl_group : 0;
     if (lanes > 8) return false;
-    for (const Tri *t : {&a, &b})
-        if ((double)t->n > kAutoClusterRowsPerLevel * (double)t->nlev) return false;
+    if (!narrow(a) || !narrow(b)) return false;
     return tile_plan(a, elem, lanes, stream) && tile_plan(b, elem, lanes, stream);
 }
 
@@ -436,12 +437,12 @@ void Handle::apply_precond(const T *d_r, T *d_z, const KState *stp) {
     timed(PC_VEC, (double)v * n, [&] { fill_sentinel_st<T>(y, n, stp, stream); });
     timed(PC_FWD, tri_bytes(Lf, v, 2), [&] {
         sweep_st<T>(Lf, Lval.as<T>(), SW_FWD_DIV, d_r, nullptr, nullptr, y, nullptr, ticket(), err(), stp, stream,
-                    swcfg, use_inv_diag ? invL.as<T>() : nullptr);
+                    free_cfg(Lf), use_inv_diag ? invL.as<T>() : nullptr);
     });
     timed(PC_VEC, (double)v * n, [&] { fill_sentinel_st<T>(d_z, n, stp, stream); });
     timed(PC_BWD, tri_bytes(Ltb, v, 3), [&] {
         sweep_st<T>(Ltb, Ltval.as<T>(), SW_BWD_IC, nullptr, y, Dvec.as<T>(), d_z, nullptr, ticket() + 1, err(), stp,
-                    stream, swcfg, (const T *)nullptr);
+                    stream, free_cfg(Ltb), (const T *)nullptr);
     });
 }
 
@@ -525,7 +526,7 @@ int Handle::solve(int method, double conv_cri, int max_ite, double normB, const 
         } else {
             fill_sentinel_st<T>(t1, n, nullptr, s);
             sweep_st<T>(Lf, Cval.as<T>(), SW_FWD_DIV, r, nullptr, nullptr, t1, nullptr, ticket(), err(), nullptr, s,
-                        swcfg, use_inv_diag ? invC.as<T>() : nullptr);
+                        free_cfg(Lf), use_inv_diag ? invC.as<T>() : nullptr);
         }
         std::swap(r, t1);
     }
@@ -652,11 +653,11 @@ int Handle::solve(int method, double conv_cri, int max_ite, double normB, const 
                 timed(PC_VEC, nv, [&] { fill_sentinel_st<T>(u, n, st, s); });
                 timed(PC_BWD, tri_bytes(Ub, vb, 2), [&] {
                     sweep_st<T>(Ub, Uval.as<T>(), SW_BWD_DIV, r, nullptr, nullptr, u, nullptr, ticket(), err(), st, s,
-                                swcfg, use_inv_diag ? invU.as<T>() : nullptr);
+                                free_cfg(Ub), use_inv_diag ? invU.as<T>() : nullptr);
                 });
                 timed(PC_VEC, nv, [&] { fill_sentinel_st<T>(t1, n, st, s); });
                 timed(PC_FWD, tri_bytes(Lf, vb, 4), [&] {
-                    sweep_st<T>(Lf, Cval.as<T>(), SW_FWD_EIS, r, u, nullptr, t1, w, ticket() + 1, err(), st, s, swcfg,
+                    sweep_st<T>(Lf, Cval.as<T>(), SW_FWD_EIS, r, u, nullptr, t1, w, ticket() + 1, err(), st, s, free_cfg(Lf),
                                 use_inv_diag ? invC.as<T>() : nullptr);
                 });
             }

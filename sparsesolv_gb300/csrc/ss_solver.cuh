@@ -102,8 +102,8 @@ struct Handle {
     SweepCfg swcfg;
     int fac_backoff_ns = 0;
     bool use_inv_diag = true;
-    int sweep_mode = 0;            // 0 auto (default), 1 sync-free, 2 cluster, 3 neighbour-synchronised cluster,
-                                   // 4 push (one cluster, no cluster-wide barrier; IC pair)
+    int sweep_mode = 0;            // 0 auto (default: tile, else sync-free), 1 sync-free, 2 cluster,
+                                   // 3 neighbour-synchronised cluster, 4 push (one cluster, IC pair)
     unsigned long long fac_epoch = 0;  // bumped whenever the factor values change (push records refill)
     int batch_group = 0;           // lanes a row in the sweeps of the owning C handle's internal batch (0: auto)
     int spmv_group_req = 0;        // lanes a row in the SpMV (0: from the row-length distribution)
@@ -123,11 +123,11 @@ struct Handle {
     int cl_group = 4;              // lanes per row in the cluster sweep
     // ic: an IC sweep (the only kind the neighbour-synchronised plan serves)
     bool cluster_ok(Tri &t, size_t elem, bool ic);
+    SweepCfg free_cfg(const Tri &t) const;  // the sync-free sweep's launch shape
     bool push_ok(size_t elem);  // both triangles of the IC pair
     bool tile_ok(Tri &a, Tri &b, size_t elem);  // the whole-GPU tile sweeps serve both triangles
-    // the automatic mode may take the push sweep (off in the standalone batches: their
-    // instances' bits must not depend on which schedule a batch's size leads to, and the
-    // lane-summed schedules give the same bits at the same lanes a row)
+    // the automatic mode may sum rows by age (off in the standalone batches, whose persistent
+    // engine and launches give the same bits: both sum by lanes)
     bool push_auto = true;
 
     Prof prof;
