@@ -30,7 +30,8 @@
 //   curl-curl, real:  10^3  54 / 55 [221 / 222], 20^3 124 / 126 [496 / 501],
 //                     41^3 371 / 359 [1,095 / 1,090], 80^3 1,079 / 1,023 [2,237 / 2,195] (push)
 //   SGS pair, 48^3:   490 / 483 [1,834 / 1,810] (lockstep)
-//   eddy currents:    33^3 727 / 906 [1,638 / 1,525], 60^3 1,526 / 1,839 [3,616 / 3,338] (lockstep)
+//   eddy currents:    33^3 640 / 813 [1,638 / 1,525], 60^3 1,310 / 1,668 [3,616 / 3,338] (lockstep); 707 / 903 and
+//                     1,490 / 1,830 with a lane holding both parts of a sum and 2.5 times fewer tiles
 //   FP32, 44^3:       206 / 210 [504 / 498] (push)
 //
 // Every wait is bounded (the handle's spin limit) and ends early when the error
@@ -262,41 +263,67 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                     } while (!__all_sync(0xffffffffu, have));
                     return x;
                 };
-                T res = Sc<T>::zero(), u0 = res;
                 int row = 0;
-                bool lead;  // this lane has the row's result
-                if (LANES > 0) {
-                    const int r = lane / LANES;
-                    lead = lane % LANES == 0 && r < cnt;
-                    T b0 = Sc<T>::zero(), lv = b0;
+                bool lead;  // this lane has the row's result (or a component of it)
+                if constexpr (LANES > 0) {
+                    // Lanes 2 l and 2 l + 1 hold the real and the imaginary part of entry lane l's sum. The arithmetic is
+                    // that of k_sweep on complex values, a component a lane: the forward right-hand side starts lane 0's
+                    // sum, the IC pair's values come negated.
+                    using R = typename Sc<T>::real;
+                    constexpr int W = 2 * LANES;  // GPU lanes a row
+                    const int r = lane / W, el = lane >> 1;
+                    const bool im = lane & 1;
+                    lead = lane % W < 2 && r < cnt;
+                    auto part = [&](T q) { return im ? q.y : q.x; };
+                    // components of a * b and of acc + a * b: p, q the parts of b that a.x and a.y meet
+                    auto cmul = [&](T f, R p, R q) { return mul_rn(f.x, p) + (im ? mul_rn(f.y, q) : -mul_rn(f.y, q)); };
+                    auto cmadd = [&](R s, T f, R p, R q) {
+                        if constexpr (sizeof(R) == 8) return fma(im ? f.y : -f.y, q, fma(f.x, p, s));
+                        else return s + cmul(f, p, q);
+                    };
+                    R b0 = R(0), ua = R(0);
+                    T lv = Sc<T>::zero();
+                    if (lead) row = ((const int *)(rec + 16 * (of.w & 0xffff)))[r];
+                    if (r < cnt) lv = ((const T *)(rec + 16 * ((unsigned)of.w >> 16)))[r];
                     if (lead) {
-                        row = ((const int *)(rec + 16 * (of.w & 0xffff)))[r];
-                        lv = ((const T *)(rec + 16 * ((unsigned)of.w >> 16)))[r];
-                        if (MODE != SW_BWD_IC) b0 = rhs[row];
-                        if (MODE == SW_BWD_IC || MODE == SW_FWD_EIS) u0 = aux[row];
+                        if (MODE != SW_BWD_IC) b0 = part(rhs[row]);
+                        if (MODE == SW_BWD_IC || MODE == SW_FWD_EIS) ua = part(aux[row]);
                     }
-                    // the arithmetic of k_sweep: the forward right-hand side starts lane 0's sum, the IC pair's values
-                    // come negated
-                    T acc = MODE == SW_FWD_DIV ? b0 : Sc<T>::zero();
-                    const unsigned short *c = (const unsigned short *)(rec + 16 * (of.y & 0xffff)) + lane;
-                    v += lane;
+                    R acc = MODE == SW_FWD_DIV ? b0 : R(0);
+                    const unsigned short *c = (const unsigned short *)(rec + 16 * (of.y & 0xffff)) + el;
+                    v += el;
 #pragma unroll 1
                     for (int k = 0; k < nb; ++k) {
                         const int2 w = need[k];
                         const int cc = c[32 * k];
                         const T vv = v[32 * k];
                         wait_for(w.x, w.y);
-                        acc = madd(acc, vv, cfar ? value(cc, cfar + 32 * k + lane) : X[cc]);
+                        const T xx = cfar ? value(cc, cfar + 32 * k + el) : X[cc];
+                        acc = cmadd(acc, vv, im ? xx.y : xx.x, im ? xx.x : xx.y);
                     }
 #pragma unroll
-                    for (int m = LANES / 2; m >= 1; m >>= 1) acc = acc + Sc<T>::shfl_xor(acc, m);
-                    if (MODE == SW_BWD_IC) res = madd(u0, lv, acc);
-                    else if (MODE == SW_FWD_DIV) res = acc * lv;
-                    else if (MODE == SW_FWD_EIS) res = ((b0 - u0) - acc) * lv;
-                    else res = (b0 - acc) * lv;
+                    for (int m = LANES / 2; m >= 1; m >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, 2 * m);
+                    R num = acc;
+                    if (MODE == SW_FWD_EIS) num = (b0 - ua) - acc;
+                    else if (MODE == SW_BWD_DIV) num = b0 - acc;
+                    const R other = __shfl_xor_sync(0xffffffffu, num, 1);
+                    // num.x and num.y as they meet lv.x and lv.y
+                    R mine;
+                    if (MODE == SW_BWD_IC) mine = cmadd(ua, lv, num, other);
+                    else {
+                        const T nm = im ? T{other, num} : T{num, other};
+                        mine = cmul(nm, part(lv), im ? lv.x : lv.y);
+                    }
                     wait_for(nd.z, nd.w);  // the own-ring slots are free
-                    if (lead) X[(h0.z + r) & (L.S_own - 1)] = res;
+                    if (lead) ((R *)(X + ((h0.z + r) & (L.S_own - 1))))[im] = mine;
+                    __syncwarp();
+                    if (lane == 0) tl_st_release(prog + 4u * warp, g + TS_W);
+                    if (lead) {
+                        tl_give((R *)(out + row) + im, mine);
+                        if (MODE == SW_FWD_EIS) ((R *)(out2 + row))[im] = mine + ua;
+                    }
                 } else {
+                    T res, u0 = Sc<T>::zero();
                     const int k1 = (h0.x >> 16) & 15, k2 = (h0.x >> 20) & 15;
                     lead = lane < cnt;  // lane r has row r outside the columns
                     // what the row starts from: on its way while the first block waits
@@ -388,12 +415,12 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                         }
                     }
                     if (lead) X[(h0.z + lane) & (L.S_own - 1)] = res;
-                }
-                __syncwarp();
-                if (lane == 0) tl_st_release(prog + 4u * warp, g + TS_W);
-                if (lead) {
-                    tl_give(out + row, res);
-                    if (MODE == SW_FWD_EIS) out2[row] = res + u0;
+                    __syncwarp();
+                    if (lane == 0) tl_st_release(prog + 4u * warp, g + TS_W);
+                    if (lead) {
+                        tl_give(out + row, res);
+                        if (MODE == SW_FWD_EIS) out2[row] = res + u0;
+                    }
                 }
             }
         } else if (warp < TS_W + TS_R) {

@@ -39,9 +39,10 @@ TileLayout tile_layout(int elem) {
 
 // More tiles put fewer rows of a level on an SM, each border costs its latency once. Measured best (us a forward sweep):
 // 2,430 rows 1 tile 48, 2 tiles 51; 21,660 rows 8 tiles 116, 16 120; 196,800 rows 32-64 tiles 364, 100 375; 1,497,840 rows
-// 152 tiles 1,124, 300 1,048. 0.014 n^0.7 is 3, 15, 71 and 294.
-int tile_count(int n) {
-    const int t = (int)std::lround(0.014 * std::pow((double)n, 0.7));
+// 152 tiles 1,124, 300 1,048. 0.014 n^0.7 is 3, 15, 71 and 294. Groups by lanes hold few rows, and want more tiles: complex
+// 101,376 rows 44 tiles 820, 110 643, 152 622; 626,580 rows 155 tiles 1,947, 300 1,432, 400 1,310.
+int tile_count(int n, int lanes) {
+    const int t = (int)std::lround((lanes ? 0.035 : 0.014) * std::pow((double)n, 0.7));
     return std::max(1, std::min(t, n));
 }
 
@@ -96,7 +97,7 @@ void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
         }
     }
     std::vector<int> gfirst;
-    const int most = C.lanes ? 32 / C.lanes : 32;  // rows of a group
+    const int most = C.lanes ? 16 / C.lanes : 32;  // rows of a group (by lanes two GPU lanes an entry lane)
     for (int q = 0; q < nr;) {
         const int l = C.level[C.row(rows[q])];
         int e = q;
@@ -351,7 +352,7 @@ TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, con
         return P;
     };
     if (n <= 0) return fail("no rows");
-    if (T <= 0) T = tile_count(n);
+    if (T <= 0) T = tile_count(n, lanes);
     T = std::min(T, n);
     P.T = T;
     P.lay = lay ? *lay : tile_layout(elem);

@@ -20,7 +20,9 @@
 //   * by lanes (complex values): lane q of `lanes` sums every lanes-th entry from q
 //     in column order, a step of one entry a lane waiting for what it reads, then a
 //     butterfly: the arithmetic of the cluster and sync-free sweeps, bit for bit.
-//     The iterates of the singular complex systems are sensitive to rounding.
+//     The iterates of the singular complex systems are sensitive to rounding. Two
+//     GPU lanes share a lane's sum, one its real and one its imaginary part, which
+//     halves the FP64 instructions between a dependency and the row's result.
 // Both depend on the row alone and not on how rows fall into tiles and groups.
 //
 // Values a group reads come from two shared-memory rings: the tile's own values
@@ -59,7 +61,8 @@ struct TileLayout {
 };
 TileLayout tile_layout(int elem);
 
-// One group's record, staged with one bulk copy. Lanes of a row are r * G .. r * G + G - 1 in the columns, r in the tails;
+// One group's record, staged with one bulk copy. Lanes of a row are r * G .. r * G + G - 1 in the columns, r in the tails
+// (by lanes: entry lane l is GPU lanes 2 l and 2 l + 1, and only 16 entry lanes are used);
 // every array of values or codes holds all 32 lanes (padding lanes and columns: value 0, the ring slot that holds zero),
 // so the kernel's loads have constant strides and no bounds.
 //   [0]   16 ints: {cnt | lg G << 8 | K1 << 16 | K2 << 20, blocks | has far entries << 16, first own slot,
@@ -112,7 +115,7 @@ struct TilePlanHost {
     std::vector<long long> rec_off;               // per tile, bytes
 };
 
-int tile_count(int n);
+int tile_count(int n, int lanes);
 // n rows: prp/pci the level-ordered rows (columns as row ids, the diagonal included), ipos[row] position of a row,
 // level[row]; lower: solve order is ascending rows. lanes: 0 sums by age, 4 or 8 by lanes. T tiles (<= 0: tile_count).
 TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level,

@@ -68,7 +68,7 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
             const int nb = hd[1] & 0xffff, blk = lanes ? 1 : 4;
             const bool far = (hd[1] >> 16) != 0;
             const TileRec R = tile_rec(cnt, nb, blk, far, kt[1] + kt[2], 8);
-            if (cnt < 1 || cnt * G > 32) return bad("group shape", t, g, cnt);
+            if (cnt < 1 || cnt * G > (lanes ? 16 : 32)) return bad("group shape", t, g, cnt);
             if (R.size != 16 * gm[1] || 16 * gm[2] + R.size > L.B_rec) return bad("record size", t, g, R.size);
             // the staging ring: whoever's bytes it takes must be done, and the barrier slot free
             const Span me{16 * gm[2], 16 * gm[2] + R.size};
