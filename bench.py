@@ -72,10 +72,9 @@ NCU_FP64_PIPE = {
 
 
 def sweep_kind(mode, cplx):
-    """The sweep schedule a mode runs: the automatic mode (0) takes the push sweep for real values and the
-    one-cluster lockstep sweep for complex ones, where their plans fit."""
+    """The sweep schedule a mode runs: the automatic mode (0) takes the tile sweep, for real and complex values."""
     if mode == 0:
-        return "cluster" if cplx else "push"
+        return "tile"
     return {1: "sync-free", 2: "cluster", 3: "neighbour", 4: "push"}.get(mode, "cluster")
 
 
@@ -110,9 +109,10 @@ def parse():
                     help="lanes a row in the sweeps of the handle's internal batch (mixed precision, --rhs); 0 auto")
     ap.add_argument("--batch-sizes", default="8,32",
                     help="cfg4: the range of N (voxels a side) of the 256 systems, N ~ U{lo..hi}")
-    ap.add_argument("--batch-persistent", action=argparse.BooleanOptionalAction, default=True,
+    ap.add_argument("--batch-persistent", action=argparse.BooleanOptionalAction, default=None,
                     help="cfg4: FP64 ICCG starts with one CTA per instance running all its iterations where every "
-                         "instance is small enough (the default); --no-batch-persistent: launches per phase")
+                         "instance is small enough; --no-batch-persistent: launches per phase; default: the "
+                         "library's rule on the batch's rows a level")
     ap.add_argument("--sweep-mode", type=int, default=0, choices=[0, 1, 2, 3, 4],
                     help="triangular sweeps: 0 automatic, 1 sync-free, 2 one-cluster level-synchronous, "
                          "3 one-cluster neighbour-synchronised, 4 one-cluster push")
@@ -525,8 +525,8 @@ def run_ours(args):
                      "launch_ms": dms / max(dlaunch, 1), "launches": dlaunch,
                      "fp64_pipe_frac": None if K > 1 else NCU_FP64_PIPE.get((args.workload, args.precision, sweep_kind(
                          tuned["mode"] if tuned else args.sweep_mode, np.iscomplexobj(val)), dom)),
-                     "limit": "dependency levels swept one after another on one 16-SM cluster (about 1,400 at 80^3): "
-                              "FP64 latency and issue on those SMs and cross-SM latency, not HBM bandwidth"},
+                     "limit": "dependency levels swept one after another (about 1,400 at 80^3): FP64 and shared-memory "
+                              "latency of a level, and the hand-over between SMs, not HBM bandwidth"},
         "kernel_ms_per_step": {k: v[0] / args.steps for k, v in stats.items()},
         "clocks": clk, "host_s": t_host,
     }
@@ -700,7 +700,8 @@ def run_batch(args):
         systems.append(case.assemble(coils_list=coils))
     bt = _capi.Batch(local)
     bt.set_precision(_capi.PREC_MIXED if args.precision == "mixed" else _capi.PREC_FP64)
-    bt.set_persistent(args.batch_persistent)
+    if args.batch_persistent is not None:
+        bt.set_persistent(args.batch_persistent)
     for rp, ci, va, B in systems:
         bt.add(rp, ci, va, B)
     inst = sum(len(B) for _, _, _, B in systems)
@@ -794,7 +795,8 @@ def run_batch(args):
         "config": {"workload": "256 curl-curl systems, N ~ U{%d..%d} voxels, 4 coil right-hand sides each" % (lo, hi),
                    "iterations_engine": "persistent (one CTA per instance) where every instance has at most "
                                         "16,384 rows, else launches per phase" if args.batch_persistent
-                   else "launches per phase (CUDA graphs)",
+                   else "launches per phase (CUDA graphs)" if args.batch_persistent is not None
+                   else "automatic (persistent where the batch's levels are wide, else launches per phase)",
                    "instances": total_inst, "rows": int(sum(len(B) * (len(rp) - 1) for rp, _, _, B in systems)),
                    "method": "shifted ICCG", "alpha": ALPHA, "tolerance": TOL, "converged": conv_all,
                    "sweep_schedule": "autotuned: %s" % json.dumps(tuned) if tuned else "fixed (8 lanes a row)",
@@ -838,7 +840,8 @@ def batch_measure(local, sizes, persistent, steps=2):
         bt = _capi.Batch(local)
         try:
             bt.set_precision(_capi.PREC_MIXED if prec == "mixed" else _capi.PREC_FP64)
-            bt.set_persistent(persistent)
+            if persistent is not None:
+                bt.set_persistent(persistent)
             for rp, ci, va, B in systems:
                 bt.add(rp, ci, va, B)
             bt.start(_capi.METHOD_ICCG, ALPHA, conv=TOL, max_ite=MAXIT)

@@ -507,7 +507,8 @@ class Batch:
         self._check(self.lib.ssg_batch_set_graphs(self.b, 1 if on else 0), "ssg_batch_set_graphs")
 
     def set_persistent(self, on):
-        """FP64 ICCG starts with one CTA per instance running all of its iterations (small systems)."""
+        """FP64 ICCG starts with one CTA per instance running all of its iterations (small systems); without a call the
+        batch's rows a level decide."""
         self._check(self.lib.ssg_batch_set_persistent(self.b, 1 if on else 0), "ssg_batch_set_persistent")
 
     def autotune(self):

@@ -1009,7 +1009,11 @@ bool Batch::persist_ok() const {
     if ((int)h_sys_tile.size() != S + 1) return false;
     for (int q = 0; q < S; ++q)
         if (h_sys_tile[q + 1] - h_sys_tile[q] > PERSIST_MAX_TILES) return false;
-    return true;
+    // Mean rows of a level at which the persistent engine overtakes the launches. Measured, ms a batch, persistent / launches:
+    // 1.2-4k rows an instance, 64 instances (1.0k rows a level) 20.9 / 14.9, 256 (4k) 27.8 / 16.7, 1,024 (16k) 40.8 / 37.8;
+    // 4-15k rows, 256 (7k) 107 / 51, 1,024 (30k) 155 / 184.
+    constexpr double wide = 24576.0;
+    return persist == PERSIST_ON || (double)h.n >= wide * (double)h.Lf.nlev;
 }
 
 // each instance's rows of each level of the forward and backward triangles: within a

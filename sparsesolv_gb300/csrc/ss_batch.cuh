@@ -47,6 +47,8 @@ struct OState {
     double normB, norm, scale, pad;
 };
 
+enum : int { PERSIST_OFF = 0, PERSIST_ON = 1, PERSIST_AUTO = 2 };
+
 struct BatchSystem {
     int n = 0, nnz = 0, nrhs = 1;
     std::vector<int> rp, ci;
@@ -122,9 +124,10 @@ struct Batch {
     static constexpr int GRAPH_ITERS = 8;
     bool use_graphs = true;
     // persistent ICCG (one CTA per instance runs all its iterations, ss_batch.cu): used
-    // for FP64 ICCG starts when on (the default) and every instance has at most 8 tiles;
-    // the same bits as the launches, 1.24x their speed on 1,024 instances of 1-4k rows
-    bool persist = true;
+    // for FP64 ICCG starts when on and every instance has at most 8 tiles; the same bits as
+    // the launches. By default (PERSIST_AUTO) where the batch's levels are wide enough to
+    // fill the GPU with instances
+    int persist = PERSIST_AUTO;
     std::vector<int> h_sys_tile;        // host copy of the first tile of each instance
     DBuf d_pl_f, d_pr_f, d_pl_b, d_pr_b;  // per-instance level ranges of the forward / backward triangles
     uint64_t pr_key = ~0ull;            // pattern the ranges were made for

@@ -673,7 +673,7 @@ int ssg_batch_set_graphs(ssg_batch bd, int enable) {
 int ssg_batch_set_persistent(ssg_batch bd, int enable) {
     return bguarded(bd, [&](ssg::Batch &b) {
         if (b.running) return SSG_ERR_STATE;
-        b.persist = enable != 0;
+        b.persist = enable ? ssg::PERSIST_ON : ssg::PERSIST_OFF;
         return SSG_OK;
     });
 }

@@ -255,7 +255,8 @@ def test_autotuned_batch_meets_the_bar_and_stays_deterministic(gpu, oracle, syst
 def _persist_run(persist, systems, Bs):
     bt = _capi.Batch(0)
     try:
-        bt.set_persistent(persist)
+        if persist is not None:
+            bt.set_persistent(persist)
         for (rp, ci, va, _), B in zip(systems, Bs):
             bt.add(rp, ci, va, B)
         bt.start(_capi.METHOD_ICCG, ALPHA, conv=1e-8, max_ite=5000)
@@ -295,3 +296,26 @@ def test_persistent_batch_same_bits_as_launches(gpu, oracle):
     got2, _ = _persist_run(True, systems2, Bs2)
     for k in range(3):
         assert np.array_equal(got2[k][0], ref2[k][0]) and np.array_equal(got2[k][1], ref2[k][1])
+
+
+@pytest.mark.parametrize("rows,count", [(16000, 4), (16000, 3), (16384, 3)])
+def test_automatic_engine_same_bits_either_side_of_its_line(gpu, rows, count):
+    """Without set_persistent the engine follows the batch's rows a level (24,576). Block-diagonal
+    systems of two levels put the batch above it (4 x 16,000 rows, 3 x 16,384: at the line) and below."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(rows + count)
+    systems, Bs = [], []
+    for _ in range(count):
+        off = np.zeros(rows - 1)
+        off[::2] = rng.uniform(-0.9, -0.1, rows // 2)
+        A = sp.diags([off, rng.uniform(1.0, 2.0, rows), off], [-1, 0, 1]).tocsr()
+        A.eliminate_zeros()
+        b = A @ rng.standard_normal(rows)
+        systems.append((A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data, b))
+        Bs.append(b[None])
+    ref, ref_logs = _persist_run(False, systems, Bs)
+    got, got_logs = _persist_run(None, systems, Bs)
+    for k in range(count):
+        assert got[k][3].all() if np.ndim(got[k][3]) else got[k][3]
+        assert np.array_equal(got[k][0], ref[k][0]) and np.array_equal(got[k][1], ref[k][1])
+        assert np.array_equal(got_logs[k][0], ref_logs[k][0])
