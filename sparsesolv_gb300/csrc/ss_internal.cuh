@@ -86,7 +86,7 @@ struct PushPlan {
 struct TilePlan {
     bool ready = false, failed = false;
     int n = -1, nnz = -1, nlev = -1;  // shape of the triangle the plan was made for
-    int T = 0, lanes = 0;             // tiles; how rows are summed
+    int T = 0, CS = 1, lanes = 0;     // tiles, of a cluster; how rows are summed
     TileLayout lay{};
     DBuf tiles, groups, halo, rel;    // ss_tile_plan.hpp
     DBuf rec, dval, dlv;              // the records; values refilled when the factor's values change

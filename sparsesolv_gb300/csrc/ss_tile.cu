@@ -9,33 +9,43 @@
 // because tiles only depend on lower tiles, the latency of a border is paid once
 // per border and not once per level.
 //
-// A CTA claims tiles in order through a ticket (every wait is on a tile some
-// running CTA holds) and runs three kinds of warps:
+// By age, 8 consecutive tiles run on one thread-block cluster and store what they
+// solve into the rings of the cluster's CTAs that read it (st.relaxed.cluster): a
+// border inside the cluster costs a store into another SM and a poll of the own
+// shared memory in place of a store to memory and polls of the L2. The first lap of
+// a ring is filled that way, whose slots the CTA marks unsolved before the cluster's
+// barrier lets anyone start; later laps and other clusters' values come from memory.
+//
+// A cluster claims its tiles in order through a ticket (every wait is on a tile some
+// running cluster holds, or of the same cluster) and its CTAs run three kinds of warps:
 //   * compute warps take the tile's groups round robin (group g: warp g % TS_W),
 //     sum, write the values to the own ring, publish their progress and store the
-//     values to memory;
+//     values to the cluster's readers and to memory;
 //   * receiver warps bring the halo in, 32 values a chunk: each lane polls the
 //     output vector for one value (a sentinel marks the unsolved) and puts it into
-//     the halo ring; the count of values here, in list order, is published;
+//     the halo ring, or polls the ring for a value the cluster stores there; the
+//     count of values here, in list order, is published;
 //   * one warp stages the groups' records with bulk copies as ring space frees.
 // Waits inside a CTA are one load of the progress words and one vote.
-// Values go between CTAs through the output vector alone: an aligned 4- or 8-byte
-// store is single-copy atomic, so a value is its own flag and no fence is needed.
+// Values go between CTAs one aligned 4- or 8-byte store at a time, which is
+// single-copy atomic, so a value is its own flag and no fence is needed.
 //
 // What bounds it: the chain of dependency levels (1,410 forward at 80^3), not bytes
 // (1 % of HBM) and not yet FP64: an FP64 instruction holds its warp for 64 cycles
 // and an SM issues one in 19, so a group's 12-15 instructions set the split of the
 // sums. Measured on a GB300, microseconds a sweep (forward / backward), with the
 // one-cluster schedules this replaces as the automatic choice in brackets:
-//   curl-curl, real:  10^3  54 / 55 [221 / 222], 20^3 124 / 126 [496 / 501],
-//                     41^3 371 / 359 [1,095 / 1,090], 80^3 1,079 / 1,023 [2,237 / 2,195] (push)
+//   curl-curl, real:  10^3  54 / 55 [221 / 222], 20^3 120 / 123 [496 / 501],
+//                     41^3 322 / 325 [1,095 / 1,090], 80^3 908 / 904 [2,237 / 2,195] (push); without clusters 123 / 127,
+//                     375 / 379 and 1,101 / 994
 //   SGS pair, 48^3:   490 / 483 [1,834 / 1,810] (lockstep)
 //   eddy currents:    33^3 640 / 813 [1,638 / 1,525], 60^3 1,310 / 1,668 [3,616 / 3,338] (lockstep); 707 / 903 and
 //                     1,490 / 1,830 with a lane holding both parts of a sum and 2.5 times fewer tiles
 //   FP32, 44^3:       206 / 210 [504 / 498] (push)
 //
 // Every wait is bounded (the handle's spin limit) and ends early when the error
-// word is set; the CTA then drains its copies and leaves.
+// word is set; the CTA then drains its copies and only goes along to the cluster's
+// barriers, until its cluster leaves together.
 #include <algorithm>
 
 #include "sparsesolv_gb300.h"
@@ -109,6 +119,30 @@ __device__ __forceinline__ void tl_give(cplxf *p, cplxf v) {
 }
 
 // a warp that tests a staged group's barrier has itself taken the group staged there before, so the parity is unambiguous
+// CTAs of a cluster: a value stored into another one's shared memory, and barriers of all
+__device__ __forceinline__ unsigned tl_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned tl_mapa(unsigned a, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void tl_send(unsigned a, int v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void tl_send(unsigned a, float v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(unsent(v)) : "memory");
+}
+__device__ __forceinline__ void tl_send(unsigned a, double v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(unsent(v)) : "memory");
+}
+__device__ __forceinline__ void tl_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
 static_assert(TS_NM % TS_W == 0, "groups of one barrier belong to one warp");
 static_assert(TS_TAILS == 2 && TS_W < 32, "the stages and progress words below");
 
@@ -138,7 +172,7 @@ __device__ __forceinline__ void tl_vals(const cplxf *b, int lane, cplxf (&v)[4])
 }
 
 struct TileArgs {
-    int T;
+    int T, CS;
     const int4 *tiles, *groups;
     const int *halo, *rel;
     const unsigned char *rec;
@@ -171,7 +205,8 @@ struct Bound {
 };
 
 // LANES: 0 sums by age, 4 or 8 by lanes (ss_tile_plan.hpp)
-template <typename T, int MODE, int LANES>
+// CL: clusters of several CTAs
+template <typename T, int MODE, int LANES, bool CL>
 __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
     if (a.st && !a.st->active) return;
     extern __shared__ __align__(16) unsigned char tl_smem[];
@@ -187,18 +222,37 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
     const unsigned long long lim = spin_limit_ns(a.err);
     constexpr int EB = (int)sizeof(T);
     bool bad = false;
+    const int CS = CL ? a.CS : 1, rank = CL ? (int)tl_rank() : 0;
+    const unsigned ring = sbase + (unsigned)L.o_x + (unsigned)(L.S_own * EB);  // the halo ring, here and in the other CTAs
 
     if (tid == 0) X[L.S_own + L.S_halo] = Sc<T>::zero();
-    for (;;) {
-        // ---- next tile
-        if (tid == 0) s_tile = atomicAdd(a.ticket, 1);
+    const bool once = a.T <= (int)gridDim.x;  // as many CTAs as tiles: each takes one
+    for (bool first = true;; first = false) {
+        // ---- next CS tiles, one a CTA
+        int t = 0;
+        if (tid == 0 && rank == 0 && (first || !CL)) t = atomicAdd(a.ticket, 1) * CS;
+        if (!CL) {
+            if (tid == 0) s_tile = t;
+        } else {
+            tl_cluster_sync();  // no CTA of the cluster stores into this one's ring any more
+            if (rank == 0 && tid == 0) {
+                // not before all of the cluster are done: another cluster may be free earlier (80^3: 966 us instead of 911)
+                if (!first) t = *(volatile int *)a.err ? a.T : atomicAdd(a.ticket, 1) * CS;
+                for (int q = 0; q < CS; ++q) tl_send(tl_mapa((unsigned)__cvta_generic_to_shared(&s_tile), q), t);
+            }
+            // slots of the first lap unsolved
+            for (int q = tid; q < L.S_halo * EB / 16; q += TS_THREADS)
+                ((uint4 *)(X + L.S_own))[q] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        }
         if (tid < TS_NM) tl_mbar_init(full + 8u * tid, 1);
         if (tid < 32) ((volatile int *)(tl_smem + L.o_prog))[tid] = tid < TS_W ? tid : 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        __syncthreads();
-        const int tile = s_tile;
-        if (tile >= a.T) break;
-        const int4 td = a.tiles[tile];
+        if (!CL) __syncthreads();
+        else tl_cluster_sync();
+        if (s_tile >= a.T) break;
+        const int tile = s_tile + rank;
+        // a CTA without a tile goes along to the barriers, and so does one that gave up
+        const int4 td = tile < a.T && !bad ? a.tiles[tile] : make_int4(0, 0, 0, 0);
         const int ng = td.y, nch = td.w;
         int issued = 0;  // groups staged
 
@@ -240,7 +294,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                 const unsigned char *rec = record(g);
                 if (!rec) break;
                 const int4 *hd = (const int4 *)rec;
-                const int4 h0 = hd[0], nd = hd[1], of = hd[3];
+                const int4 h0 = hd[0], nd = hd[1], hp = hd[2], of = hd[3];
                 const int cnt = h0.x & 0xff, lg = (h0.x >> 8) & 0xff;
                 const int nb = h0.y & 0xffff;
                 const int *cfar = (h0.y >> 16) ? (const int *)(rec + 16 * of.z) : nullptr;
@@ -265,6 +319,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                 };
                 int row = 0;
                 bool lead;  // this lane has the row's result (or a component of it)
+                // who else reads the row: the first two ahead, as the record is given back with the result
+                const int *push = (const int *)(rec + 16 * hp.y);
+                int to0 = -1, to1 = -1;
+                auto send = [&](int to, auto val, int comp) {
+                    if (CL && to >= 0)
+                        tl_send(tl_mapa(ring + (unsigned)((to & 0xfffff) * EB + comp), (unsigned)to >> 20), val);
+                };
                 if constexpr (LANES > 0) {
                     // Lanes 2 l and 2 l + 1 hold the real and the imaginary part of entry lane l's sum. The arithmetic is
                     // that of k_sweep on complex values, a component a lane: the forward right-hand side starts lane 0's
@@ -286,6 +347,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                     if (lead) row = ((const int *)(rec + 16 * (of.w & 0xffff)))[r];
                     if (r < cnt) lv = ((const T *)(rec + 16 * ((unsigned)of.w >> 16)))[r];
                     if (lead) {
+                        if (CL && hp.x > 0) to0 = push[r];
+                        if (CL && hp.x > 1) to1 = push[32 + r];
                         if (MODE != SW_BWD_IC) b0 = part(rhs[row]);
                         if (MODE == SW_BWD_IC || MODE == SW_FWD_EIS) ua = part(aux[row]);
                     }
@@ -316,9 +379,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                     }
                     wait_for(nd.z, nd.w);  // the own-ring slots are free
                     if (lead) ((R *)(X + ((h0.z + r) & (L.S_own - 1))))[im] = mine;
+                    for (int k = 2; CL && k < hp.x; ++k)
+                        if (lead) send(push[32 * k + r], mine, im * (int)sizeof(R));
                     __syncwarp();
                     if (lane == 0) tl_st_release(prog + 4u * warp, g + TS_W);
                     if (lead) {
+                        send(to0, mine, im * (int)sizeof(R));
+                        send(to1, mine, im * (int)sizeof(R));
                         tl_give((R *)(out + row) + im, mine);
                         if (MODE == SW_FWD_EIS) ((R *)(out2 + row))[im] = mine + ua;
                     }
@@ -329,6 +396,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                     // what the row starts from: on its way while the first block waits
                     T b0 = Sc<T>::zero(), lv = b0;
                     if (lead) {
+                        if (CL && hp.x > 0) to0 = push[lane];
+                        if (CL && hp.x > 1) to1 = push[32 + lane];
                         row = ((const int *)(rec + 16 * (of.w & 0xffff)))[lane];
                         if (MODE != SW_BWD_IC) {
                             lv = ((const T *)(rec + 16 * ((unsigned)of.w >> 16)))[lane];
@@ -415,9 +484,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                         }
                     }
                     if (lead) X[(h0.z + lane) & (L.S_own - 1)] = res;
+                    for (int k = 2; CL && k < hp.x; ++k)
+                        if (lead) send(push[32 * k + lane], res, 0);
                     __syncwarp();
                     if (lane == 0) tl_st_release(prog + 4u * warp, g + TS_W);
                     if (lead) {
+                        send(to0, res, 0);
+                        send(to1, res, 0);
                         tl_give(out + row, res);
                         if (MODE == SW_FWD_EIS) out2[row] = res + u0;
                     }
@@ -436,13 +509,15 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                 const int reln = ch + TS_R < nch ? a.rel[td.z + ch + TS_R] : -1;
                 // the slots' previous values are dead (they are, long since, unless the halo ring is full)
                 if (rel >= 0) wait_for(rel, 0);
-                bool have = j < 0, head = false;
+                bool have = j == -1, head = false;
+                const bool pushed = CL && j == -2;
+                T *const slot = X + L.S_own + ((32 * ch + lane) & (L.S_halo - 1));
                 int told = 0, tries = 0;
                 Bound b(a.err, lim);
                 while (!bad) {
                     T x;
-                    if (!have && tl_take(out + j, x)) {
-                        X[L.S_own + ((32 * ch + lane) & (L.S_halo - 1))] = x;
+                    if (!have && (pushed ? tl_take(slot, x) : tl_take(out + j, x))) {
+                        if (!pushed) *slot = x;
                         have = true;
                     }
                     const unsigned miss = ~__ballot_sync(0xffffffffu, have);
@@ -456,7 +531,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                     if (told == 32) break;
                     if (__any_sync(0xffffffffu, b.spent(63))) bad = true;
                     // far ahead of the producers: poll gently
-                    if (++tries > 16) __nanosleep(100);
+                    if (++tries > 16 && __any_sync(0xffffffffu, !have && !pushed)) __nanosleep(100);
                 }
                 if (bad) break;
                 j = jn;
@@ -490,6 +565,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                            gtimer() - t0 < 1000000ull) {
                     }
                 }
+            if (!CL) return;
+            bad = true;  // the whole CTA goes on to the cluster's barriers and leaves with it
+        }
+        if (once) {
+            if (CL) tl_cluster_sync();
             return;
         }
         if (tid < TS_NM) tl_mbar_inval(full + 8u * tid);
@@ -552,7 +632,7 @@ bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s) {
     SSG_CUDA(cudaMemcpyAsync(level.data(), T.level.p, sizeof(int) * T.n, cudaMemcpyDeviceToHost, s));
     SSG_CUDA(cudaStreamSynchronize(s));
     const TilePlanHost H =
-        tile_plan_host(T.n, T.nlev, prp.data(), pci.data(), ipos.data(), level.data(), T.lower, elem, lanes, 0);
+        tile_plan_host(T.n, T.nlev, prp.data(), pci.data(), ipos.data(), level.data(), T.lower, elem, lanes, 0, tile_cluster(tile_count(T.n, lanes), lanes));
     if (!H.ok) {
         P.failed = true;
         return false;
@@ -575,6 +655,7 @@ bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s) {
     SSG_CUDA(cudaStreamSynchronize(s));
     P.lay = H.lay;
     P.T = H.T;
+    P.CS = H.CS;
     P.key_val = P.key_lv = nullptr;
     P.key_epoch = ~0ull;
     P.ready = true;
@@ -613,6 +694,7 @@ void sweep_tile(Tri &tri, const T *val, int mode, const T *rhs, const T *aux, co
     }
     TileArgs a;
     a.T = P.T;
+    a.CS = P.CS;
     a.tiles = P.tiles.as<int4>();
     a.groups = P.groups.as<int4>();
     a.halo = P.halo.as<int>();
@@ -626,31 +708,46 @@ void sweep_tile(Tri &tri, const T *val, int mode, const T *rhs, const T *aux, co
     a.st = st;
     a.err = err;
     a.L = P.lay;
-    const int grid = std::min(P.T, tile_sms());
-#define SSG_TS(M, LN)                                                                                          \
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = P.CS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(TS_THREADS);
+    cfg.dynamicSmemBytes = P.lay.total;
+    cfg.stream = s;
+    cfg.gridDim = dim3(std::min((P.T + P.CS - 1) / P.CS, std::max(1, tile_sms() / P.CS)) * P.CS);
+#define SSG_TS(M, LN, CL)                                                                                      \
     do {                                                                                                       \
-        auto kern = k_sweep_tile<T, M, LN>;                                                                    \
+        auto kern = k_sweep_tile<T, M, LN, CL>;                                                                \
         static bool prepared = false;                                                                          \
         if (!prepared) {                                                                                       \
             SSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX));    \
             prepared = true;                                                                                   \
         }                                                                                                      \
-        kern<<<grid, TS_THREADS, P.lay.total, s>>>(a);                                                         \
+        SSG_CUDA(cudaLaunchKernelEx(&cfg, kern, a));                                                           \
     } while (0)
-#define SSG_TM(LN)                                                \
-    switch (mode) {                                               \
-        case SW_FWD_DIV: SSG_TS(SW_FWD_DIV, LN); break;           \
-        case SW_BWD_IC: SSG_TS(SW_BWD_IC, LN); break;             \
-        /* by age the same arithmetic on the other triangle */    \
-        case SW_BWD_DIV: SSG_TS((LN ? SW_BWD_DIV : SW_FWD_DIV), LN); break; \
-        default: SSG_TS(SW_FWD_EIS, LN); break;                   \
+#define SSG_TM(LN, CL)                                                     \
+    switch (mode) {                                                        \
+        case SW_FWD_DIV: SSG_TS(SW_FWD_DIV, LN, CL); break;                \
+        case SW_BWD_IC: SSG_TS(SW_BWD_IC, LN, CL); break;                  \
+        /* by age the same arithmetic on the other triangle */             \
+        case SW_BWD_DIV: SSG_TS((LN ? SW_BWD_DIV : SW_FWD_DIV), LN, CL); break; \
+        default: SSG_TS(SW_FWD_EIS, LN, CL); break;                        \
     }
     if constexpr (!by_lanes) {
-        SSG_TM(0)
+        if (P.CS > 1) {
+            SSG_TM(0, true)
+        } else {
+            SSG_TM(0, false)
+        }
     } else if (P.lanes == 4) {
-        SSG_TM(4)
+        SSG_TM(4, false)
     } else {
-        SSG_TM(8)
+        SSG_TM(8, false)
     }
 #undef SSG_TM
 #undef SSG_TS

@@ -11,15 +11,19 @@
 #include <cstring>
 #include <deque>
 #include <exception>
+#include <memory>
 #include <thread>
 
 namespace ssg {
 
-TileLayout tile_layout(int elem) {
+TileLayout tile_layout(int elem, int lanes) {
     TileLayout L{};
-    // 32 KB each for the own and the halo ring whatever the value size; the rest stages records
-    L.S_own = 32 * 1024 / elem;
-    L.S_halo = 32 * 1024 / elem;
+    // By age 16 KB for the own ring and 64 KB for the halo ring, whose first lap the cluster's other tiles store into: a tile
+    // reads about twice as many rows of other tiles as it has. Measured, us a forward sweep at 41^3 and 80^3 with 32 + 32 KB
+    // 347, 1,050; 32 + 64 326, 949; 16 + 64 324, 927; 16 + 128 (too little is left for records) 350, 884. By lanes 32 KB each
+    // (16 + 64 KB: 33^3 640 -> 664). The rest stages records.
+    L.S_own = (lanes ? 32 : 16) * 1024 / elem;
+    L.S_halo = (lanes ? 32 : 64) * 1024 / elem;
     int o = 0;
     L.o_x = o;
     o += ts_al16((L.S_own + L.S_halo + 1) * elem);
@@ -37,14 +41,23 @@ TileLayout tile_layout(int elem) {
     return L;
 }
 
-// More tiles put fewer rows of a level on an SM, each border costs its latency once. Measured best (us a forward sweep):
-// 2,430 rows 1 tile 48, 2 tiles 51; 21,660 rows 8 tiles 116, 16 120; 196,800 rows 32-64 tiles 364, 100 375; 1,497,840 rows
-// 152 tiles 1,124, 300 1,048. 0.014 n^0.7 is 3, 15, 71 and 294. Groups by lanes hold few rows, and want more tiles: complex
-// 101,376 rows 44 tiles 820, 110 643, 152 622; 626,580 rows 155 tiles 1,947, 300 1,432, 400 1,310.
+// More tiles put fewer rows of a level on an SM, each border costs its latency once. Measured (us a forward sweep by age, in
+// clusters from 8 tiles on): 2,430 rows 1 tile 55, 3 tiles 54; 21,660 rows 8 tiles 125, 12 120, 15 120; 48,800 rows 16 168,
+// 24 159; 83,700 rows 20 227, 32 204, 40 207; 196,800 rows 36 338, 50 311, 71 321; 405,000 rows 72 494, 104 454, 128 457;
+// 626,580 rows 120 616, 160 565, 200 564; 1,497,840 rows 250 992, 304 927, 380 911, 400 911. 0.0044 n^0.8 is 2, 13, 25, 38, 75,
+// 135, 191 and 383. Groups by lanes hold few rows, and want more tiles, most so where there are few of them: complex 101,376
+// rows 44 tiles 820, 110 643, 152 622; 626,580 rows 155 tiles 1,947, 300 1,432, 400 1,310; 0.035 n^0.7 is 112 and 400.
 int tile_count(int n, int lanes) {
-    const int t = (int)std::lround((lanes ? 0.035 : 0.014) * std::pow((double)n, 0.7));
+    const int t = (int)std::lround(lanes ? 0.035 * std::pow((double)n, 0.7) : 0.0044 * std::pow((double)n, 0.8));
     return std::max(1, std::min(t, n));
 }
+
+// Tiles of a cluster. The next tiles wait for all of a cluster's, so clusters pay where most tiles run at once and a level
+// is one group's work, and cost where the GPU's tiles at a time set the pace: by lanes, with 2 to 4 rows a group, 60^3 took
+// 1,360 us with 1, 1,437 with 4 and 1,593 with 8 (33^3 664, 655, 651). By age, 1 against 8: 3 tiles 54 / 57, 20^3 123 / 120,
+// 41^3 384 / 324, 80^3 1,101 / 927; 16 gives 80^3 918 and 41^3 311 instead of 316 (50 tiles): not worth the larger clusters,
+// of which fewer fit beside other work.
+int tile_cluster(int T, int lanes) { return lanes || T < 8 ? 1 : 8; }
 
 namespace {
 
@@ -75,7 +88,67 @@ struct Scratch {
     explicit Scratch(int n) : hpos((size_t)n, -1) {}
 };
 
-void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
+// the rows of other tiles that a tile reads, in (level, order), and which of them are pushed to it
+struct Halo {
+    std::vector<int> row;
+    std::vector<unsigned char> pushed;
+    const char *why = nullptr;
+};
+
+void find_halo(const Ctx &C, int p0, int p1, Scratch &S, Halo &H) {
+    for (int p = p0; p < p1; ++p) {
+        const int i = C.row(p), t = C.ipos[i];
+        for (int k = C.prp[t]; k < C.prp[t + 1]; ++k) {
+            const int j = C.pci[k];
+            if (j == i) continue;
+            if (j < 0 || j >= C.n || C.ord(j) >= p || C.level[j] >= C.level[i]) {
+                H.why = "an entry is not a dependency of its row";
+                break;
+            }
+            if (C.ord(j) < p0 && S.hpos[j] < 0) {
+                S.hpos[j] = 0;
+                H.row.push_back(j);
+            }
+        }
+    }
+    std::sort(H.row.begin(), H.row.end(), [&](int a, int b) {
+        return C.level[a] != C.level[b] ? C.level[a] < C.level[b] : C.ord(a) < C.ord(b);
+    });
+    H.pushed.assign(H.row.size(), 0);
+    for (int h : H.row) S.hpos[h] = -1;
+}
+
+// per place of the solve order from p0 on, the ring slots of the cluster's CTAs that take its row: rank << 20 | slot
+struct Push {
+    int p0 = 0;
+    std::vector<int> ptr, dat;
+    int count(int p) const { return ptr.empty() ? 0 : ptr[p - p0 + 1] - ptr[p - p0]; }
+};
+
+// the first lap's values that tiles t0 to t1 - 1 take from each other
+template <typename F>
+void find_pushes(const Ctx &C, int t0, int t1, const F &first, std::vector<Halo> &halo, Push &P) {
+    P.p0 = first(t0);
+    P.ptr.assign((size_t)(first(t1) - P.p0) + 2, 0);
+    auto each = [&](auto f) {
+        for (int t = t0; t < t1; ++t) {
+            const int m = std::min((int)halo[t].row.size(), C.L.S_halo);
+            for (int q = 0; q < m; ++q) {
+                const int p = C.ord(halo[t].row[q]) - P.p0;
+                if (p >= 0) f(t, q, p);
+            }
+        }
+    };
+    each([&](int t, int q, int p) {
+        halo[t].pushed[q] = 1;
+        P.ptr[p + 2]++;
+    });
+    for (size_t p = 2; p < P.ptr.size(); ++p) P.ptr[p] += P.ptr[p - 1];
+    P.dat.resize((size_t)P.ptr.back());
+    each([&](int t, int q, int p) { P.dat[P.ptr[p + 1]++] = (t - t0) << 20 | q; });  // leaves ptr[p + 1] at the end of p
+}
+
+void plan_tile(const Ctx &C, int p0, int p1, const Halo &halo, const Push &pushes, Scratch &S, TileOut &O) {
     const int nr = p1 - p0, elem = C.elem;
     const TileLayout &L = C.L;
     // rows in (level, order), and groups of rows of one level
@@ -109,26 +182,7 @@ void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
     const int ng = (int)gfirst.size();
     gfirst.push_back(nr);
     // halo: the rows of other tiles read here, in (level, order)
-    std::vector<int> hal;
-    for (int q = 0; q < nr; ++q) {
-        const int i = C.row(rows[q]), t = C.ipos[i];
-        for (int k = C.prp[t]; k < C.prp[t + 1]; ++k) {
-            const int j = C.pci[k];
-            if (j == i) continue;
-            if (j < 0 || j >= C.n || C.ord(j) >= C.ord(i) || C.level[j] >= C.level[i]) {
-                O.why = "an entry is not a dependency of its row";
-                for (int h : hal) S.hpos[h] = -1;
-                return;
-            }
-            if (C.ord(j) < p0 && S.hpos[j] < 0) {
-                S.hpos[j] = 0;
-                hal.push_back(j);
-            }
-        }
-    }
-    std::sort(hal.begin(), hal.end(), [&](int a, int b) {
-        return C.level[a] != C.level[b] ? C.level[a] < C.level[b] : C.ord(a) < C.ord(b);
-    });
+    const std::vector<int> &hal = halo.row;
     const int nh = (int)hal.size(), nch = (nh + 31) / 32;
     for (int q = 0; q < nh; ++q) S.hpos[hal[q]] = q;
     // first group that needs a chunk delivered, were every halo entry read through the ring
@@ -242,7 +296,9 @@ void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
             O.why = "a row with too many entries";
             break;
         }
-        const TileRec R = tile_rec(c, nb, blk, any_far, KT, elem);
+        int KP = 0;
+        for (int r = 0; r < c; ++r) KP = std::max(KP, pushes.count(rows[q0 + r]));
+        const TileRec R = tile_rec(c, nb, blk, any_far, KT, KP, elem);
         if (R.size > L.B_rec / 2) {
             O.why = "a group's record does not fit the staging ring";
             break;
@@ -280,6 +336,8 @@ void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
             hd[2 + 2 * s] = own_need[s];
             hd[3 + 2 * s] = halo_need[s];
         }
+        hd[8] = KP;
+        hd[9] = R.o_push / 16;
         hd[12] = R.o_old / 16 | R.o_tail / 16 << 16;
         hd[13] = R.o_cold / 16 | R.o_ctail / 16 << 16;
         hd[14] = R.o_cfar / 16;
@@ -291,6 +349,11 @@ void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
         const unsigned short pad = (unsigned short)(L.S_own + L.S_halo);
         for (int q = 0; q < 32 * blk * nb; ++q) cold[q] = pad;
         for (int q = 0; q < 32 * KT; ++q) ctail[q] = pad;
+        int *push = (int *)(rec + R.o_push);
+        for (int q = 0; q < 32 * KP; ++q) push[q] = -1;
+        for (int r = 0; r < c; ++r)
+            for (int k = 0, m = pushes.count(rows[q0 + r]); k < m; ++k)
+                push[32 * k + r] = pushes.dat[pushes.ptr[rows[q0 + r] - pushes.p0] + k];
         const int e_old = (int)((base + R.o_old) / elem), e_tail = (int)((base + R.o_tail) / elem),
                   e_lv = (int)((base + R.o_lv) / elem);
         for (int r = 0; r < c; ++r) {
@@ -326,7 +389,7 @@ void plan_tile(const Ctx &C, int p0, int p1, Scratch &S, TileOut &O) {
     O.halo.assign((size_t)nch * 32, -1);
     O.rel.assign((size_t)nch, -1);
     for (int q = 0; q < nh; ++q) {
-        O.halo[q] = hal[q];
+        O.halo[q] = halo.pushed[q] ? -2 : hal[q];
         if (q >= L.S_halo) O.rel[q / 32] = std::max(O.rel[q / 32], halo_last[q - L.S_halo]);
     }
     for (int h : hal) S.hpos[h] = -1;
@@ -344,7 +407,7 @@ int plan_threads() {
 }  // namespace
 
 TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level,
-                            bool lower, int elem, int lanes, int T, const TileLayout *lay) {
+                            bool lower, int elem, int lanes, int T, int CS, const TileLayout *lay) {
     TilePlanHost P;
     auto fail = [&](const char *why) {
         P.ok = false;
@@ -355,37 +418,51 @@ TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, con
     if (T <= 0) T = tile_count(n, lanes);
     T = std::min(T, n);
     P.T = T;
-    P.lay = lay ? *lay : tile_layout(elem);
+    P.CS = CS = std::max(1, CS);
+    P.lay = lay ? *lay : tile_layout(elem, lanes);
     P.dval.assign((size_t)prp[n], -1);
     P.dlv.assign((size_t)n, 0);
-    const Ctx C{n, elem, lanes, prp, pci, ipos, level, lower, P.lay, P.dval.data(), P.dlv.data()};
-    std::vector<TileOut> out((size_t)T);
     auto first = [&](int t) { return (int)((long long)n * t / T); };
-    {
-        const int nt = std::max(1, std::min(plan_threads(), T));
-        std::atomic<int> next{0};
-        std::vector<std::exception_ptr> errs((size_t)nt);
-        auto work = [&](int q) {
-            try {
-                Scratch S(n);
-                for (int t; (t = next.fetch_add(1)) < T;) plan_tile(C, first(t), first(t + 1), S, out[t]);
-            } catch (...) {
-                errs[q] = std::current_exception();
+    // three passes over tiles, clusters and tiles again, their items taken one at a time by a few host threads
+    const int nt = std::max(1, std::min(plan_threads(), T)), NC = (T + CS - 1) / CS;
+    const int items[3] = {T, CS > 1 ? NC : 0, T};
+    std::vector<Halo> halo((size_t)T);
+    std::vector<Push> push((size_t)NC);
+    std::vector<TileOut> out((size_t)T);
+    const Ctx C{n, elem, lanes, prp, pci, ipos, level, lower, P.lay, P.dval.data(), P.dlv.data()};
+    std::atomic<int> next[3] = {{0}, {0}, {0}}, done[3] = {{0}, {0}, {0}};
+    std::vector<std::exception_ptr> errs((size_t)nt);
+    auto work = [&](int q) {
+        std::unique_ptr<Scratch> S;
+        for (int pass = 0; pass < 3; ++pass) {
+            for (int t; (t = next[pass].fetch_add(1)) < items[pass]; done[pass].fetch_add(1)) {
+                try {
+                    if (!S) S.reset(new Scratch(n));
+                    if (pass == 0) find_halo(C, first(t), first(t + 1), *S, halo[t]);
+                    else if (pass == 1) find_pushes(C, t * CS, std::min(T, (t + 1) * CS), first, halo, push[t]);
+                    else if (!halo[t].why) plan_tile(C, first(t), first(t + 1), halo[t], push[t / CS], *S, out[t]);
+                } catch (...) {
+                    errs[q] = std::current_exception();
+                }
             }
-        };
-        std::vector<std::thread> pool;
-        for (int q = 1; q < nt; ++q) {
-            try {
-                pool.emplace_back(work, q);
-            } catch (...) {
-                break;  // fewer threads: the others take its tiles
-            }
+            while (done[pass].load() < items[pass]) std::this_thread::yield();
         }
-        work(0);
-        for (auto &t : pool) t.join();
-        for (auto &e : errs)
-            if (e) std::rethrow_exception(e);
+    };
+    std::vector<std::thread> pool;
+    for (int q = 1; q < nt; ++q) {
+        try {
+            pool.emplace_back(work, q);
+        } catch (...) {
+            break;  // fewer threads: the others take its items
+        }
     }
+    work(0);
+    for (auto &t : pool) t.join();
+    for (auto &e : errs)
+        if (e) std::rethrow_exception(e);
+    for (int t = 0; t < T; ++t)
+        if (halo[t].why) return fail(halo[t].why);
+    for (auto &p : push) P.npush += (int)p.dat.size();
     long long off = 0, g0 = 0, c0 = 0;
     P.tiles.resize((size_t)T * 4);
     P.rec.resize((size_t)T);

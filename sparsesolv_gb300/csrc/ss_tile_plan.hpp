@@ -30,7 +30,13 @@
 // the tile's halo list, ordered by dependency level and delivered in that order.
 // An entry whose ring slot would be reused before the read is "far": it is
 // read from the output vector in memory, in its place in the sum, where every
-// value is its own ready flag. Every wait is for an earlier group, an earlier halo value or a lower tile.
+// value is its own ready flag. Every wait is for an earlier group, an earlier
+// halo value or a lower tile.
+//
+// CS consecutive tiles run on one thread-block cluster. A halo value of the first lap
+// of the ring whose tile runs on the same cluster is not polled for in memory: the
+// row's owner stores it into the reader's ring slot, which no one else writes before
+// its readers are done.
 #pragma once
 
 #include <vector>
@@ -53,13 +59,13 @@ constexpr int TS_SMEM_MAX = 220 * 1024;   // dynamic shared memory of a CTA
 
 SSG_HD inline int ts_al16(int x) { return (x + 15) & ~15; }
 
-// Shared-memory carve-up, by value size alone.
+// Shared-memory carve-up, by value size and way of summing.
 struct TileLayout {
     int S_own, S_halo;   // ring slots (powers of two); slot S_own + S_halo holds zero (padding entries)
     int B_rec;           // bytes of the record ring
     int o_x, o_full, o_place, o_prog, o_rec, total;
 };
-TileLayout tile_layout(int elem);
+TileLayout tile_layout(int elem, int lanes);
 
 // One group's record, staged with one bulk copy. Lanes of a row are r * G .. r * G + G - 1 in the columns, r in the tails
 // (by lanes: entry lane l is GPU lanes 2 l and 2 l + 1, and only 16 entry lanes are used);
@@ -67,20 +73,22 @@ TileLayout tile_layout(int elem);
 // so the kernel's loads have constant strides and no bounds.
 //   [0]   16 ints: {cnt | lg G << 8 | K1 << 16 | K2 << 20, blocks | has far entries << 16, first own slot,
 //          columns in the first block, per tail stage, oldest first, the last own group it needs (-1: none) and the halo
-//          values it needs, offsets / 16: o_old | o_tail << 16, o_cold | o_ctail << 16, o_cfar, o_row | o_lv << 16}
+//          values it needs, KP, o_push / 16, 0, 0,
+//          offsets / 16: o_old | o_tail << 16, o_cold | o_ctail << 16, o_cfar, o_row | o_lv << 16}
 //   need  per block {last own group needed, halo values needed}; a block is four columns, or one step by lanes
 //   rows  cnt row ids
 //   lv    cnt values: 1 / L_ii or D_i
 //   old   per block its values of every lane (ts_col); tails (K1 + K2) x 32 values
 //   codes old (per block those of a lane together) and tails as unsigned shorts: ring slots, TS_FAR for a far entry
 //   cfar  with far entries: per old code the row id
+//   push  KP x 32 (by row): rank << 20 | ring slot of a CTA of the cluster that reads the row, -1
 // By age, a row's entries fill the last columns, so that a block's entries are about equally old in every row; the first
 // block's leading columns may be empty in all rows and are skipped.
 constexpr int TS_FAR = 0xFFFF;
 struct TileRec {
-    int o_need, o_row, o_lv, o_old, o_tail, o_cold, o_ctail, o_cfar, size;
+    int o_need, o_row, o_lv, o_old, o_tail, o_cold, o_ctail, o_cfar, o_push, size;
 };
-SSG_HD inline TileRec tile_rec(int cnt, int nb, int blk, bool far, int KT, int elem) {
+SSG_HD inline TileRec tile_rec(int cnt, int nb, int blk, bool far, int KT, int KP, int elem) {
     TileRec r;
     r.o_need = 64;
     r.o_row = r.o_need + ts_al16(8 * nb);
@@ -90,7 +98,8 @@ SSG_HD inline TileRec tile_rec(int cnt, int nb, int blk, bool far, int KT, int e
     r.o_cold = r.o_tail + elem * 32 * KT;
     r.o_ctail = r.o_cold + 2 * 32 * blk * nb;
     r.o_cfar = r.o_ctail + 2 * 32 * KT;
-    r.size = r.o_cfar + (far ? 4 * 32 * blk * nb : 0);
+    r.o_push = r.o_cfar + (far ? 4 * 32 * blk * nb : 0);
+    r.size = r.o_push + 4 * 32 * KP;
     return r;
 }
 // index of column q of a lane in its block's values: 16 bytes a lane at a time
@@ -101,13 +110,13 @@ SSG_HD inline int ts_col(int q, int lane, int blk, int elem) {
 
 // tiles: per tile {first group, groups, first halo chunk, halo chunks}
 // groups: per group {record offset / 16, record bytes / 16, ring offset / 16, group that must be done before the copy}
-// halo: row ids, 32 a chunk (-1: padding); rel: per 32 of them the group up to which all must be done before they are delivered (-1: none)
+// halo: row ids, 32 a chunk (-1: padding, -2: stored into its slot by a tile of the cluster); rel: per 32 of them the group up to which all must be done before they are delivered (-1: none)
 // dval: per entry of the level-ordered triangle its element index in rec, -1: the diagonal;
 // dlv: per level-ordered row the element index of its lv
 struct TilePlanHost {
     bool ok = false;
     const char *why = "";
-    int T = 0, nfar = 0;
+    int T = 0, CS = 1, nfar = 0, npush = 0;
     long long rec_bytes = 0;
     TileLayout lay{};
     std::vector<int> tiles, groups, halo, rel, dval, dlv;
@@ -116,9 +125,11 @@ struct TilePlanHost {
 };
 
 int tile_count(int n, int lanes);
+int tile_cluster(int T, int lanes);
 // n rows: prp/pci the level-ordered rows (columns as row ids, the diagonal included), ipos[row] position of a row,
-// level[row]; lower: solve order is ascending rows. lanes: 0 sums by age, 4 or 8 by lanes. T tiles (<= 0: tile_count).
+// level[row]; lower: solve order is ascending rows. lanes: 0 sums by age, 4 or 8 by lanes. T tiles (<= 0: tile_count), CS
+// of them a cluster.
 TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level,
-                            bool lower, int elem, int lanes, int T, const TileLayout *lay = nullptr);
+                            bool lower, int elem, int lanes, int T, int CS, const TileLayout *lay = nullptr);
 
 }  // namespace ssg

@@ -19,15 +19,15 @@ static std::string bad(const char *what, int tile, int g, int x) {
 // values of the triangle in its level-ordered layout, lvec per level-ordered row, rhs by row; y: the solution.
 // lay: {S_own, S_halo, B_rec} or null. Returns "" or what is wrong; stats: tiles, far entries.
 static std::string run(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level, bool lower,
-                       int lanes, int T, const int *lay, const double *val, const double *lvec, const double *rhs, double *y,
+                       int lanes, int T, int CS, const int *lay, const double *val, const double *lvec, const double *rhs, double *y,
                        int *stats) {
-    TileLayout L = tile_layout(8);
+    TileLayout L = tile_layout(8, lanes);
     if (lay) {
         L.S_own = lay[0];
         L.S_halo = lay[1];
         L.B_rec = lay[2];
     }
-    const TilePlanHost P = tile_plan_host(n, nlev, prp, pci, ipos, level, lower, 8, lanes, T, &L);
+    const TilePlanHost P = tile_plan_host(n, nlev, prp, pci, ipos, level, lower, 8, lanes, T, CS, &L);
     if (!P.ok) return std::string("no plan: ") + P.why;
     if (L.o_rec + (lay ? 0 : L.B_rec) > TS_SMEM_MAX) return "layout exceeds shared memory";
     stats[0] = P.T;
@@ -45,15 +45,26 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
     }
     std::vector<char> done((size_t)n, 0);
     int rows_seen = 0;
+    std::vector<std::vector<int>> slots((size_t)CS);  // rows pushed to each CTA of the cluster, by slot
     for (int t = 0; t < P.T; ++t) {
         const int g0 = P.tiles[4 * t], ng = P.tiles[4 * t + 1], c0 = P.tiles[4 * t + 2], nch = P.tiles[4 * t + 3];
         std::vector<int> own_row, own_grp;           // by production position
         std::vector<std::vector<int>> own_rd, halo_rd((size_t)nch * 32);  // groups that read each value from its ring
         std::vector<int> need3((size_t)ng), hneed((size_t)ng, 0);
+        if (t % CS == 0)
+            for (auto &v : slots) v.assign((size_t)L.S_halo, -1);
+        std::vector<int> hrow((size_t)nch * 32);
         for (int c = 0; c < nch * 32; ++c) {
-            const int j = P.halo[(size_t)c0 * 32 + c];
+            int j = P.halo[(size_t)c0 * 32 + c];
+            if (j == -2) {
+                j = c < L.S_halo ? slots[t % CS][c] : -1;
+                if (j < 0) return bad("a halo value is not pushed", t, c, j);
+            } else if (c < L.S_halo && slots[t % CS][c] >= 0) {
+                return bad("a push nobody reads", t, c, j);
+            }
+            hrow[c] = j;
             if (j >= 0 && !done[j]) return bad("a halo value of a later tile", t, c, j);
-            if (c && j >= 0 && level[j] < level[P.halo[(size_t)c0 * 32 + c - 1]]) return bad("halo order", t, c, j);
+            if (c && j >= 0 && level[j] < level[hrow[c - 1]]) return bad("halo order", t, c, j);
         }
         struct Span { int o, e; };
         std::vector<Span> span;
@@ -67,7 +78,7 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
             const int kt[3] = {0, (hd[0] >> 16) & 15, (hd[0] >> 20) & 15};
             const int nb = hd[1] & 0xffff, blk = lanes ? 1 : 4;
             const bool far = (hd[1] >> 16) != 0;
-            const TileRec R = tile_rec(cnt, nb, blk, far, kt[1] + kt[2], 8);
+            const TileRec R = tile_rec(cnt, nb, blk, far, kt[1] + kt[2], hd[8], 8);
             if (cnt < 1 || cnt * G > (lanes ? 16 : 32)) return bad("group shape", t, g, cnt);
             if (R.size != 16 * gm[1] || 16 * gm[2] + R.size > L.B_rec) return bad("record size", t, g, R.size);
             // the staging ring: whoever's bytes it takes must be done, and the barrier slot free
@@ -97,7 +108,7 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
             }
             need3[g] = own_w[TS_TAILS - 1];
             if (hd[12] != (R.o_old / 16 | R.o_tail / 16 << 16) || hd[13] != (R.o_cold / 16 | R.o_ctail / 16 << 16) ||
-                hd[14] != R.o_cfar / 16 || hd[15] != (R.o_row / 16 | R.o_lv / 16 << 16))
+                hd[14] != R.o_cfar / 16 || hd[9] != R.o_push / 16 || hd[15] != (R.o_row / 16 | R.o_lv / 16 << 16))
                 return bad("record offsets", t, g, 0);
             std::vector<double> res((size_t)cnt);
             for (int i = 0; i < cnt; ++i) {
@@ -117,10 +128,10 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
                     // halo: the newest chunk the waits let through; none newer may have come (checked below)
                     int q = -1;
                     for (int p = code - L.S_own; p < halo_w[s] && p < 32 * nch; p += L.S_halo)
-                        if (P.halo[(size_t)c0 * 32 + p] >= 0) q = p;  // padding lanes write nothing
+                        if (hrow[p] >= 0) q = p;  // padding lanes write nothing
                     if (q < 0) why = bad("halo value not waited for", t, g, code);
                     else halo_rd[q].push_back(g);
-                    return q < 0 ? 0.0 : y[P.halo[(size_t)c0 * 32 + q]];
+                    return q < 0 ? 0.0 : y[hrow[q]];
                 };
                 double s0 = 0.0;
                 for (int q = 0; q < blk * nb; ++q)
@@ -142,6 +153,14 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
                 if (!why.empty()) return why;
                 res[i] = v;
             }
+            for (int k = 0; k < 32 * hd[8]; ++k) {
+                const int w = ((const int *)(r + R.o_push))[k];
+                if (w < 0) continue;
+                const int to = w >> 20, slot = w & 0xfffff;
+                if (k % 32 >= cnt || to <= t % CS || to >= CS || t - t % CS + to >= P.T || slot >= L.S_halo || slots[to][slot] >= 0)
+                    return bad("push", t, g, w);
+                slots[to][slot] = rid[k % 32];
+            }
             for (int i = 0; i < cnt; ++i) {
                 y[rid[i]] = res[i];
                 own_row.push_back(rid[i]);
@@ -157,7 +176,7 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
             for (int u : own_rd[q])
                 if (u > need3[own_grp[q + L.S_own]]) return bad("own slot rewritten too early", t, own_grp[q + L.S_own], u);
         // halo ring: likewise for a chunk's delivery, and no chunk waits for a group that needs it
-        for (int q = 0; q + L.S_halo < nch * 32 && P.halo[(size_t)c0 * 32 + q + L.S_halo] >= 0; ++q)
+        for (int q = 0; q + L.S_halo < nch * 32 && hrow[q + L.S_halo] >= 0; ++q)
             for (int u : halo_rd[q])
                 if (u > P.rel[(size_t)c0 + (q + L.S_halo) / 32]) return bad("halo slot rewritten too early", t, u, q);
         for (int g = 0, run = 0; g < ng; ++g) {
@@ -170,9 +189,9 @@ static std::string run(int n, int nlev, const int *prp, const int *pci, const in
 }
 
 extern "C" const char *tile_check(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level,
-                                  int lower, int lanes, int T, const int *lay, const double *val, const double *lvec,
+                                  int lower, int lanes, int T, int CS, const int *lay, const double *val, const double *lvec,
                                   const double *rhs, double *y, int *stats) {
     static std::string why;
-    why = run(n, nlev, prp, pci, ipos, level, lower != 0, lanes, T, lay, val, lvec, rhs, y, stats);
+    why = run(n, nlev, prp, pci, ipos, level, lower != 0, lanes, T, CS, lay, val, lvec, rhs, y, stats);
     return why.c_str();
 }

@@ -69,7 +69,8 @@ SMALL = (64, 128, 32768)   # own ring, halo ring, staging ring (bytes)
 @pytest.mark.parametrize("T", [0, 1, 7, 40])
 @pytest.mark.parametrize("lay", [None, SMALL])
 @pytest.mark.parametrize("lanes", [0, 4, 8])
-def test_tile_plan_checks_and_emulates(lib, oracle, name, lower, T, lay, lanes):
+@pytest.mark.parametrize("CS", [1, 8])
+def test_tile_plan_checks_and_emulates(lib, oracle, name, lower, T, lay, lanes, CS):
     A = matrix(name)
     A.sort_indices()
     rp, ci = A.indptr.astype(np.int32), A.indices.astype(np.int32)
@@ -92,7 +93,7 @@ def test_tile_plan_checks_and_emulates(lib, oracle, name, lower, T, lay, lanes):
     y = np.full(n, np.nan)
     stats = np.zeros(2, np.int32)
     ring = None if lay is None else np.array(lay, np.int32)
-    why = lib.tile_check(n, int(nlev), _p(prp), _p(pci), _p(ipos), _p(level), int(lower), lanes, T, _p(ring), _p(val), _p(lvec),
+    why = lib.tile_check(n, int(nlev), _p(prp), _p(pci), _p(ipos), _p(level), int(lower), lanes, T, CS, _p(ring), _p(val), _p(lvec),
                          _p(r), _p(y), _p(stats)).decode()
     if "newest dependency left its ring" in why:  # another sweep serves it; never with the shipped rings here
         assert lay is not None and lanes == 0
