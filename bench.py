@@ -53,19 +53,23 @@ MAXIT = 20000
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the dominant kernel, from one ncu
-# capture of the same workload: profiles/k_sweep_push_80cube.md (push sweeps, the automatic mode's choice for
-# real values), profiles/k_sweep_cluster_80cube.md (lockstep cluster sweeps) and profiles/k_sweep_fwd_80cube.md
-# (sync-free forward sweep)
+# capture of the same workload: profiles/k_sweep_tile_80cube.md (tile sweeps, the automatic mode's choice),
+# profiles/k_sweep_push_80cube.md (push sweeps), profiles/k_sweep_cluster_80cube.md (lockstep cluster sweeps) and
+# profiles/k_sweep_fwd_80cube.md (sync-free forward sweep)
 NCU_TRAFFIC = {
+    ("cfg2", "fp64", "tile", "forward sweep"): 615.1e6,
+    ("cfg2", "fp64", "tile", "backward sweep"): 616.6e6,
     ("cfg2", "fp64", "push", "forward sweep"): 434.4e6,
     ("cfg2", "fp64", "push", "backward sweep"): 434.3e6,
     ("cfg2", "fp64", "cluster", "forward sweep"): 348.7e6,
     ("cfg2", "fp64", "cluster", "backward sweep"): 347.6e6,
     ("cfg2", "fp64", "sync-free", "forward sweep"): 360.6e6,
 }
-# the same captures' FP64 pipe (sm__inst_executed_pipe_fp64, % of peak sustained on the active SMs, averaged over
-# all 152): the push sweep runs level by level on one 16-SM cluster, bound by FP64 latency and issue on those SMs
+# the same captures' FP64 pipe (sm__inst_executed_pipe_fp64, % of peak sustained on the active SMs): the tile sweep is
+# bound by the chain of its levels, the push sweep by FP64 latency and issue on the 16 SMs of one cluster
 NCU_FP64_PIPE = {
+    ("cfg2", "fp64", "tile", "forward sweep"): 0.141,
+    ("cfg2", "fp64", "tile", "backward sweep"): 0.141,
     ("cfg2", "fp64", "push", "forward sweep"): 0.237,
     ("cfg2", "fp64", "push", "backward sweep"): 0.245,
 }
