@@ -72,6 +72,10 @@ struct Ready<cplxf> {
 
 constexpr int SW_THREADS = 128;
 constexpr int SW_U = 4;  // entries a lane polls at a time
+// Mean rows of a level above which k_sweep_wide is the faster. Measured on batches at 8 lanes a row, us a forward sweep,
+// k_sweep / k_sweep_wide: 7,300 rows a level 1,139 / 2,477, 8,600 920 / 1,890, 17,400 1,592 / 1,963: the one grows with the
+// rows, the other hardly. At 58,000 (1,024 instances of 8 to 32 voxels) a whole pass took 1,033 / 683 ms.
+constexpr double SW_WIDE = 22528.0;
 
 // One warp takes 32 / G consecutive positions. Rows of one warp may depend on each other, so no row waits alone: the warp
 // goes round one loop in which every lane polls the entries it still misses, and a row whose entries are all here is
@@ -196,14 +200,105 @@ __global__ void __launch_bounds__(SW_THREADS) k_sweep(int n, const int *__restri
     }
 }
 
+// Levels so wide that hardly an entry is waited for: a lane adds an entry as soon as it is here, with the loads of a whole
+// CTA's rows in flight. The same sums, so the same bits.
+template <typename T>
+__device__ __forceinline__ T wait_value(const T *p, int *err, int backoff_ns) {
+    T v;
+    if (Ready<T>::ok(p, v)) return v;
+    const unsigned long long start = gtimer();
+    int polls = 0;
+    while (!Ready<T>::ok(p, v)) {
+        if (backoff_ns) __nanosleep(backoff_ns);
+        if ((++polls & 31) == 0) {
+            if (*(volatile int *)err) return Ready<T>::nan();
+            if (gtimer() - start > spin_limit_ns(err)) {
+                atomicExch(err, ERR_TIMEOUT);
+                return Ready<T>::nan();
+            }
+        }
+    }
+    return v;
+}
+
+template <typename T, int G, int MODE>
+__global__ void __launch_bounds__(SW_THREADS) k_sweep_wide(int n, const int *__restrict__ perm, const int *__restrict__ prp,
+                                                      const int *__restrict__ pci, const T *__restrict__ val,
+                                                      const T *rhs, const T *aux, const T *D, T *out, T *out2,
+                                                      int *ticket, int *err, const KState *st, const T *dinv,
+                                                      int backoff_ns, const int *row_inst, const int *act,
+                                                      int act_stride) {
+    if (st && !st->active) return;
+    constexpr int ROWS = SW_THREADS / G;
+    __shared__ int s_base;
+    const int g = threadIdx.x / G;
+    const int gl = threadIdx.x % G;
+    // the value vector the sweep polls: the forward result (y) for FWD_EIS, out otherwise
+    T *poll = out;
+    for (;;) {
+        if (threadIdx.x == 0) s_base = atomicAdd(ticket, ROWS);
+        __syncthreads();
+        const int base = s_base;
+        __syncthreads();
+        if (base >= n) return;
+        const int t = base + g;
+        const int r = t < n ? perm[t] : 0;
+        // a batch skips the rows of instances that have ended (nothing of another instance reads them)
+        if (t < n && (!row_inst || act[(size_t)row_inst[r] * act_stride])) {
+            const int a = prp[t], e = prp[t + 1];
+            const bool fwd = (MODE == SW_FWD_DIV || MODE == SW_FWD_EIS);
+            const int ob = fwd ? a : a + 1;       // off-diagonal range (empty when the row is)
+            const int oe = fwd ? (e > a ? e - 1 : a) : e;
+            const int dpos = fwd ? e - 1 : a;     // diagonal position
+            // IC pair: the sum is taken negated, and the forward right-hand side starts
+            // lane 0's sum, so the row's result is one operation after the reduction
+            constexpr bool neg = (MODE == SW_FWD_DIV || MODE == SW_BWD_IC);
+            T acc = (MODE == SW_FWD_DIV && gl == 0) ? rhs[r] : Sc<T>::zero();
+            for (int k = ob + gl; k < oe; k += G) {
+                const int c = pci[k];
+                const T v = val[k];
+                const T x = wait_value(poll + c, err, backoff_ns);
+                acc = madd(acc, neg ? -v : v, x);
+            }
+            const unsigned gm = group_mask(G);
+#pragma unroll
+            for (int m = G / 2; m >= 1; m >>= 1) acc = acc + gshfl_xor(acc, m, gm);
+            if (gl == 0) {
+                // an empty row has no divisor: the result becomes inf/NaN, never an out-of-row read.
+                // With dinv the division by the diagonal is a multiplication by its
+                // precomputed reciprocal (off the critical path; rounding within 1 ulp).
+                T res;
+                if (MODE == SW_BWD_IC) {
+                    res = madd(aux[r], D[r], acc);  // aux + D * (-sum)
+                } else if (MODE == SW_FWD_DIV) {
+                    res = dinv ? acc * dinv[r] : acc / ((e > a) ? val[dpos] : Sc<T>::zero());
+                } else {
+                    T num = rhs[r] - acc;
+                    T u = Sc<T>::zero();
+                    if (MODE == SW_FWD_EIS) {
+                        u = aux[r];
+                        num = (rhs[r] - u) - acc;
+                    }
+                    if (dinv) res = num * dinv[r];
+                    else res = num / ((e > a) ? val[dpos] : Sc<T>::zero());
+                    if (MODE == SW_FWD_EIS) out2[r] = res + u;
+                }
+                Ready<T>::publish(out + r, res);
+            }
+        }
+    }
+}
+
 template <typename T, int G>
 static void launch_sweep(const Tri &tri, const T *val, int mode, const T *rhs, const T *aux, const T *D, T *out,
                          T *out2, int *ticket, int *err, const KState *st, int grid, const T *dinv,
                          const SweepCfg &cfg, cudaStream_t s) {
     const int *perm = tri.perm.as<int>(), *prp = tri.prp.as<int>(), *pci = tri.pci.as<int>();
-#define SSG_SW(M)                                                                                                 \
-    k_sweep<T, G, M><<<grid, SW_THREADS, 0, s>>>(tri.n, perm, prp, pci, val, rhs, aux, D, out, out2, ticket, err, \
-                                                 st, dinv, cfg.backoff_ns, cfg.row_inst, cfg.act, cfg.act_stride)
+    const bool wide = (double)tri.n > SW_WIDE * (double)tri.nlev;
+#define SSG_SW(M)                                                                                              \
+    (wide ? k_sweep_wide<T, G, M> : k_sweep<T, G, M>)<<<grid, SW_THREADS, 0, s>>>(                             \
+        tri.n, perm, prp, pci, val, rhs, aux, D, out, out2, ticket, err, st, dinv, cfg.backoff_ns, cfg.row_inst, \
+        cfg.act, cfg.act_stride)
     switch (mode) {
         case SW_FWD_DIV: SSG_SW(SW_FWD_DIV); break;
         case SW_BWD_IC: SSG_SW(SW_BWD_IC); break;

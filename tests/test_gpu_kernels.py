@@ -206,3 +206,30 @@ def test_switching_sweep_modes_replans(handle):
         assert np.array_equal(z3, z2) and np.array_equal(z3, z3b)
     finally:
         handle.set_tuning(_capi.TUNE_SWEEP_MODE, 0)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n", [45056, 45058, 60001])
+def test_sync_free_sweep_of_wide_levels(handle, oracle, n, cplx):
+    """Two dependency levels of n / 2 rows, at and above the line (22,528 rows a level) where the wide-level
+    sync-free kernel takes over, against the oracle's substitution: a row has one off-diagonal entry at most, so
+    the sums agree to a few roundings."""
+    rng = np.random.default_rng(n)
+    off = np.zeros(n - 1, np.complex128 if cplx else np.float64)
+    k = len(off[::2])
+    off[::2] = rng.uniform(-0.9, -0.1, k) + (1j * rng.uniform(0.1, 0.3, k) if cplx else 0)
+    A = sp.diags([off, rng.uniform(1.5, 2.0, n), off], [-1, 0, 1]).tocsr()
+    A.eliminate_zeros()
+    A.sort_indices()
+    handle.set_matrix(A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data.astype(off.dtype))
+    lrp, lci, lval, D = handle.factor(1.1)
+    r = rng.standard_normal(n) + (1j * rng.standard_normal(n) if cplx else 0)
+    try:
+        handle.set_tuning(_capi.TUNE_SWEEP_MODE, 1)
+        z = handle.apply_precond(r)
+        z2 = handle.apply_precond(r)
+    finally:
+        handle.set_tuning(_capi.TUNE_SWEEP_MODE, 0)
+    zo = oracle.ic_apply(lrp, lci, lval, D, r)
+    assert np.linalg.norm(z - zo) <= 1e-14 * np.linalg.norm(zo)
+    assert np.array_equal(z, z2)
