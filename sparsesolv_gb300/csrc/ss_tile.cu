@@ -256,10 +256,14 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
         const int ng = td.y, nch = td.w;
         int issued = 0;  // groups staged
 
-        // own groups up to og are done and h halo values are here
+        // own groups up to og are done and h halo values are here. Lane w acquires what warp w released; the vote says that
+        // all are here but orders no memory (CUDA promises that of __syncwarp alone), so the barrier is what lets every lane
+        // read, or overwrite, what another lane acquired.
         auto ready = [&](int og, int h) {
             const int want = lane < TS_W ? og + 1 : lane == TS_W ? h : 0;
-            return __all_sync(0xffffffffu, tl_ld_acquire(prog + 4u * lane) >= want) != 0;
+            const bool ok = __all_sync(0xffffffffu, tl_ld_acquire(prog + 4u * lane) >= want) != 0;
+            if (ok) __syncwarp();
+            return ok;
         };
         auto wait_for = [&](int og, int h) {
             if (ready(og, h)) return;
