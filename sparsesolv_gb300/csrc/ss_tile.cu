@@ -635,8 +635,10 @@ bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s) {
     SSG_CUDA(cudaMemcpyAsync(ipos.data(), T.ipos.p, sizeof(int) * T.n, cudaMemcpyDeviceToHost, s));
     SSG_CUDA(cudaMemcpyAsync(level.data(), T.level.p, sizeof(int) * T.n, cudaMemcpyDeviceToHost, s));
     SSG_CUDA(cudaStreamSynchronize(s));
+    const TileLimits lim = tile_limits(lanes);
     const TilePlanHost H =
-        tile_plan_host(T.n, T.nlev, prp.data(), pci.data(), ipos.data(), level.data(), T.lower, elem, lanes, 0, tile_cluster(tile_count(T.n, lanes), lanes));
+        tile_plan_host(T.n, T.nlev, prp.data(), pci.data(), ipos.data(), level.data(), T.lower, elem, lanes, 0,
+                       tile_cluster(tile_count(T.n, lanes), lanes), nullptr, &lim);
     if (!H.ok) {
         P.failed = true;
         return false;

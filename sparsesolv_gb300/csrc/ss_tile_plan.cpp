@@ -59,6 +59,19 @@ int tile_count(int n, int lanes) {
 // of which fewer fit beside other work.
 int tile_cluster(int T, int lanes) { return lanes || T < 8 ? 1 : 8; }
 
+// Consecutive rows make good tiles where a row's dependencies are near it in the order: a breadth-first or banded order, a
+// grid's natural one. In an order that scatters them a tile reads rows of most lower tiles, 32 (a chunk) at a time in level
+// order at about 0.4 us by age and 1 us by lanes, and a triangle of few levels is soon through without tiles: the sync-free
+// sweep takes about 1.3 us a level (complex 2). Measured, us a sweep forward, tiles / sync-free, by halo chunks a level of the
+// tile with most. By age, rows in random order: curl-curl 10^3 0.8 34 / 68, 12^3 1.7 47 / 78, 14^3 3.1 61 / 77, 16^3 4.8
+// 111 / 82, 20^3 8.8 226 / 84, 24^3 14 324 / 86; 27-point 16^3 2.1 40 / 61, 28^3 11 172 / 71; 7-point 16^3 5.6 29 / 26, 40^3 18
+// 95 / 35. (Breadth-first curl-curl orders have 0.2, natural grids up to 0.6.) By lanes: 9^3 0.9 88 / 108, 10^3 1.3 104 / 110,
+// 11^3 1.6 133 / 117, 16^3 3.9 254 / 136, 24^3 7.7 459 / 147. Far entries are polled in memory one by one on a row's chain:
+// orders shuffled within a window have few chunks and many of them. Far entries a row, us tiles / sync-free, complex 24^3 with
+// windows of 500, 2,000 and 6,000 rows: 0.04 1,459 / 1,712, 0.6 1,653 / 1,306, 3.7 1,574 / 734; real 40^3: 0.01 896 / 1,986,
+// 0.08 1,537 / 1,739, 0.07 1,713 / 1,328.
+TileLimits tile_limits(int lanes) { return {lanes ? 1.0 : 3.0, 0.1}; }
+
 namespace {
 
 struct TileOut {
@@ -407,7 +420,8 @@ int plan_threads() {
 }  // namespace
 
 TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level,
-                            bool lower, int elem, int lanes, int T, int CS, const TileLayout *lay) {
+                            bool lower, int elem, int lanes, int T, int CS, const TileLayout *lay,
+                            const TileLimits *lim) {
     TilePlanHost P;
     auto fail = [&](const char *why) {
         P.ok = false;
@@ -432,15 +446,29 @@ TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, con
     const Ctx C{n, elem, lanes, prp, pci, ipos, level, lower, P.lay, P.dval.data(), P.dlv.data()};
     std::atomic<int> next[3] = {{0}, {0}, {0}}, done[3] = {{0}, {0}, {0}};
     std::vector<std::exception_ptr> errs((size_t)nt);
+    // a limit passed: the passes run out without work. Each limit is on a maximum or a sum, so the outcome does not depend on
+    // the threads.
+    std::atomic<const char *> over{nullptr};
+    std::atomic<long long> nfar{0};
+    const double max_chunks = lim ? lim->chunks_per_level * std::max(nlev, 1) : 0.0;
+    const double max_far = lim ? lim->far_per_row * n : 0.0;
     auto work = [&](int q) {
         std::unique_ptr<Scratch> S;
         for (int pass = 0; pass < 3; ++pass) {
             for (int t; (t = next[pass].fetch_add(1)) < items[pass]; done[pass].fetch_add(1)) {
                 try {
+                    if (over.load()) continue;
                     if (!S) S.reset(new Scratch(n));
-                    if (pass == 0) find_halo(C, first(t), first(t + 1), *S, halo[t]);
-                    else if (pass == 1) find_pushes(C, t * CS, std::min(T, (t + 1) * CS), first, halo, push[t]);
-                    else if (!halo[t].why) plan_tile(C, first(t), first(t + 1), halo[t], push[t / CS], *S, out[t]);
+                    if (pass == 0) {
+                        find_halo(C, first(t), first(t + 1), *S, halo[t]);
+                        if (lim && (double)((halo[t].row.size() + 31) / 32) > max_chunks)
+                            over = "a tile reads too many rows of others";
+                    } else if (pass == 1) {
+                        find_pushes(C, t * CS, std::min(T, (t + 1) * CS), first, halo, push[t]);
+                    } else if (!halo[t].why) {
+                        plan_tile(C, first(t), first(t + 1), halo[t], push[t / CS], *S, out[t]);
+                        if (lim && (double)(nfar += out[t].nfar) > max_far) over = "too many far entries";
+                    }
                 } catch (...) {
                     errs[q] = std::current_exception();
                 }
@@ -462,6 +490,7 @@ TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, con
         if (e) std::rethrow_exception(e);
     for (int t = 0; t < T; ++t)
         if (halo[t].why) return fail(halo[t].why);
+    if (over.load()) return fail(over.load());
     for (auto &p : push) P.npush += (int)p.dat.size();
     long long off = 0, g0 = 0, c0 = 0;
     P.tiles.resize((size_t)T * 4);

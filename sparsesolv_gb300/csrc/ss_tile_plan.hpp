@@ -126,10 +126,18 @@ struct TilePlanHost {
 
 int tile_count(int n, int lanes);
 int tile_cluster(int T, int lanes);
+
+// What a plan may cost before the sync-free sweep is the better choice; a plan beyond it is refused.
+struct TileLimits {
+    double chunks_per_level;  // halo chunks of the tile with most of them, over the triangle's levels
+    double far_per_row;       // far entries, over the rows
+};
+TileLimits tile_limits(int lanes);
 // n rows: prp/pci the level-ordered rows (columns as row ids, the diagonal included), ipos[row] position of a row,
 // level[row]; lower: solve order is ascending rows. lanes: 0 sums by age, 4 or 8 by lanes. T tiles (<= 0: tile_count), CS
-// of them a cluster.
+// of them a cluster. lim: null for a plan at any cost.
 TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, const int *ipos, const int *level,
-                            bool lower, int elem, int lanes, int T, int CS, const TileLayout *lay = nullptr);
+                            bool lower, int elem, int lanes, int T, int CS, const TileLayout *lay = nullptr,
+                            const TileLimits *lim = nullptr);
 
 }  // namespace ssg
