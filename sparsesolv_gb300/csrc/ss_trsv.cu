@@ -19,6 +19,7 @@
 // every wait ends; each is also bounded in time and reports ERR_TIMEOUT.
 #include "ss_internal.cuh"
 #include "ss_krylov.cuh"
+#include "ss_rules.hpp"
 
 namespace ssg {
 
@@ -72,10 +73,6 @@ struct Ready<cplxf> {
 
 constexpr int SW_THREADS = 128;
 constexpr int SW_U = 4;  // entries a lane polls at a time
-// Mean rows of a level above which k_sweep_wide is the faster. Measured on batches at 8 lanes a row, us a forward sweep,
-// k_sweep / k_sweep_wide: 7,300 rows a level 1,139 / 2,477, 8,600 920 / 1,890, 17,400 1,592 / 1,963: the one grows with the
-// rows, the other hardly. At 58,000 (1,024 instances of 8 to 32 voxels) a whole pass took 1,033 / 683 ms.
-constexpr double SW_WIDE = 22528.0;
 
 // One warp takes 32 / G consecutive positions. Rows of one warp may depend on each other, so no row waits alone: the warp
 // goes round one loop in which every lane polls the entries it still misses, and a row whose entries are all here is
@@ -201,7 +198,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_sweep(int n, const int *__restri
 }
 
 // Levels so wide that hardly an entry is waited for: a lane adds an entry as soon as it is here, with the loads of a whole
-// CTA's rows in flight. The same sums, so the same bits.
+// CTA's rows in flight. The same sums, so the same bits. ss_rules.hpp has the line between the two.
 template <typename T>
 __device__ __forceinline__ T wait_value(const T *p, int *err, int backoff_ns) {
     T v;
@@ -294,7 +291,8 @@ static void launch_sweep(const Tri &tri, const T *val, int mode, const T *rhs, c
                          T *out2, int *ticket, int *err, const KState *st, int grid, const T *dinv,
                          const SweepCfg &cfg, cudaStream_t s) {
     const int *perm = tri.perm.as<int>(), *prp = tri.prp.as<int>(), *pci = tri.pci.as<int>();
-    const bool wide = (double)tri.n > SW_WIDE * (double)tri.nlev;
+    const bool wide = (double)tri.n > sweep_wide_rows(sizeof(typename Sc<T>::real) == 4, Sc<T>::is_complex, G,
+                                                      cfg.row_inst != nullptr) * (double)tri.nlev;
 #define SSG_SW(M)                                                                                              \
     (wide ? k_sweep_wide<T, G, M> : k_sweep<T, G, M>)<<<grid, SW_THREADS, 0, s>>>(                             \
         tri.n, perm, prp, pci, val, rhs, aux, D, out, out2, ticket, err, st, dinv, cfg.backoff_ns, cfg.row_inst, \
