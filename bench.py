@@ -116,7 +116,7 @@ def parse():
     ap.add_argument("--batch-persistent", action=argparse.BooleanOptionalAction, default=None,
                     help="cfg4: FP64 ICCG starts with one CTA per instance running all its iterations where every "
                          "instance is small enough; --no-batch-persistent: launches per phase; default: the "
-                         "library's rule on the batch's rows a level")
+                         "library's rule on the instances' sizes, levels and number")
     ap.add_argument("--sweep-mode", type=int, default=0, choices=[0, 1, 2, 3, 4],
                     help="triangular sweeps: 0 automatic, 1 sync-free, 2 one-cluster level-synchronous, "
                          "3 one-cluster neighbour-synchronised, 4 one-cluster push")
@@ -800,7 +800,7 @@ def run_batch(args):
                    "iterations_engine": "persistent (one CTA per instance) where every instance has at most "
                                         "16,384 rows, else launches per phase" if args.batch_persistent
                    else "launches per phase (CUDA graphs)" if args.batch_persistent is not None
-                   else "automatic (persistent where the batch's levels are wide, else launches per phase)",
+                   else "automatic (the library's rule on the instances)",
                    "instances": total_inst, "rows": int(sum(len(B) * (len(rp) - 1) for rp, _, _, B in systems)),
                    "method": "shifted ICCG", "alpha": ALPHA, "tolerance": TOL, "converged": conv_all,
                    "sweep_schedule": "autotuned: %s" % json.dumps(tuned) if tuned else "fixed (8 lanes a row)",

@@ -338,9 +338,10 @@ int ssg_batch_set_graphs(ssg_batch b, int enable);
  * another CTA; the same bits as the launch-per-phase iterations with the sync-free
  * sweep. Used when every system has at most 16,384 rows, the sweeps have a fixed lane
  * count (the batch default, 8) and the reciprocal diagonal is on; otherwise, and for
- * IC-MRTR and mixed precision, the launches run. 0: launches always. Without a call: where the
- * batch's levels hold about 25,000 rows or more, from where the persistent engine is the faster
- * (1,024 instances of 4-15k rows: 155 against 184 ms; 64 of them: 102 against 31). No
+ * IC-MRTR and mixed precision, the launches run. 0: launches always. Without a call: the faster
+ * of the two by a rule on the instances' sizes, levels and number (csrc/ss_rules.hpp): small
+ * instances persistent, few large ones by launches (5-point 20^2, 64 instances: 64 against 167 us
+ * an iteration; curl-curl 14^3, 64 instances: 1,880 against 860). No
  * reference counterpart (the reference solves one system per call). */
 int ssg_batch_set_persistent(ssg_batch b, int enable);
 /* Times the sweep schedules on the batch's block-diagonal matrix (as ssg_autotune:

@@ -508,7 +508,7 @@ class Batch:
 
     def set_persistent(self, on):
         """FP64 ICCG starts with one CTA per instance running all of its iterations (small systems); without a call the
-        batch's rows a level decide."""
+        instances' sizes, levels and number decide."""
         self._check(self.lib.ssg_batch_set_persistent(self.b, 1 if on else 0), "ssg_batch_set_persistent")
 
     def autotune(self):

@@ -10,6 +10,7 @@
 
 #include "ss_batch.cuh"
 #include "ss_kdev.cuh"
+#include "ss_rules.hpp"
 
 namespace ssg {
 
@@ -666,7 +667,7 @@ __global__ void __launch_bounds__(BT) k_bneg(BDev B, const T *a, T *out) {
 }
 
 // ---------------------------------------------------------------- host side
-static int bgrid(int NT) {
+static int bsms() {
     static int sms = 0;
     if (!sms) {
         int dev = 0;
@@ -674,8 +675,10 @@ static int bgrid(int NT) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 1;
     }
-    return std::max(1, std::min(NT, sms * 8));
+    return sms;
 }
+
+static int bgrid(int NT) { return std::max(1, std::min(NT, bsms() * 8)); }
 
 Batch::Batch(int dev) : h(dev) {
     // fixed lanes per row in both sweep schedules and in the SpMV: an
@@ -999,21 +1002,31 @@ void Batch::start(int method_, double alpha, double conv, int max_ite_) {
     queued = 0;
     chunk = 2;
     running = true;
+    persistent = persist_ok(sizeof(T));
     queue_chunk<T>();
 }
 
-bool Batch::persist_ok() const {
+bool Batch::persist_ok(size_t elem) {
     if (!persist || method != SSG_METHOD_ICCG || precision != SSG_PREC_FP64 || h.prof.on || !h.use_inv_diag) return false;
     const int G = h.swcfg.group;
     if (G != 4 && G != 8 && G != 16 && G != 32) return false;
-    if ((int)h_sys_tile.size() != S + 1) return false;
+    if (S == 0 || (int)h_sys_tile.size() != S + 1) return false;
     for (int q = 0; q < S; ++q)
         if (h_sys_tile[q + 1] - h_sys_tile[q] > PERSIST_MAX_TILES) return false;
-    // Mean rows of a level at which the persistent engine overtakes the launches. Measured, ms a batch, persistent / launches:
-    // 1.2-4k rows an instance, 64 instances (1.0k rows a level) 20.9 / 14.9, 256 (4k) 27.8 / 16.7, 1,024 (16k) 40.8 / 37.8;
-    // 4-15k rows, 256 (7k) 107 / 51, 1,024 (30k) 155 / 184.
-    constexpr double wide = 24576.0;
-    return persist == PERSIST_ON || (double)h.n >= wide * (double)h.Lf.nlev;
+    if (persist == PERSIST_ON) return true;
+    BatchShape b{};
+    b.instances = S;
+    b.rows = h.n;
+    b.nnz = h.nnz;
+    for (const BatchSystem &q : sys) {
+        b.max_rows = std::max(b.max_rows, (double)q.n);
+        b.max_nnz = std::max(b.max_nnz, (double)q.nnz);
+    }
+    b.levels = h.Lf.nlev;
+    b.sms = bsms();
+    b.complex_values = vtype == SSG_COMPLEX;
+    b.tiles = h.tile_ok(h.Lf, h.Ltb, elem);
+    return batch_persists(b);
 }
 
 // each instance's rows of each level of the forward and backward triangles: within a
@@ -1100,7 +1113,7 @@ void Batch::queue_persistent() {
 
 template <typename T>
 void Batch::queue_chunk() {
-    if (persist_ok()) {
+    if (persistent) {
         queue_persistent<T>();
         return;
     }

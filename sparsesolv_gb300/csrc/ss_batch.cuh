@@ -125,13 +125,13 @@ struct Batch {
     bool use_graphs = true;
     // persistent ICCG (one CTA per instance runs all its iterations, ss_batch.cu): used
     // for FP64 ICCG starts when on and every instance has at most 8 tiles; the same bits as
-    // the launches. By default (PERSIST_AUTO) where the batch's levels are wide enough to
-    // fill the GPU with instances
+    // the launches where both sum by lanes. By default (PERSIST_AUTO) where ss_rules.hpp expects it to be the faster
     int persist = PERSIST_AUTO;
+    bool persistent = false;            // the running start's engine
     std::vector<int> h_sys_tile;        // host copy of the first tile of each instance
     DBuf d_pl_f, d_pr_f, d_pl_b, d_pr_b;  // per-instance level ranges of the forward / backward triangles
     uint64_t pr_key = ~0ull;            // pattern the ranges were made for
-    bool persist_ok() const;
+    bool persist_ok(size_t elem);
     void persist_ranges();
     template <typename T>
     void queue_persistent();

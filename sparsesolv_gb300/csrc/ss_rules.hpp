@@ -2,6 +2,9 @@
 // were fitted to. Plain C++, so that a CPU test can hold them against those times.
 #pragma once
 
+#include <algorithm>
+#include <cmath>
+
 namespace ssg {
 
 // Sync-free sweep (ss_trsv.cu): mean rows of a level above which k_sweep_wide is faster than k_sweep. The one polling loop of
@@ -24,5 +27,41 @@ inline double sweep_wide_rows(bool fp32, bool complex_values, int G, bool batch)
     if (fp32 && !complex_values) return 5632.0;
     return batch ? 22528.0 : 11264.0;
 }
+
+// Batched FP64 ICCG (ss_batch.cu): one CTA an instance that runs all of its iterations, or the launches? Estimates of an
+// iteration's time in us, fitted to 325 measured batches (1 to 2,048 instances, 400 to 16,000 rows each, of curl-curl, grid,
+// banded and random systems, equal and mixed sizes); over them the engine chosen is 2 % slower than the better one on average
+// (complex 1 %), where the persistent one everywhere is 48 % (15 %) and the launches everywhere 20 % (38 %).
+//   persistent  the largest instance's levels (a barrier each), rows and entries; more instances than about a third of the SMs
+//               share SMs and memory
+//   launches    the launches, the levels of the longest instance at a cost that grows with their width up to the lane-by-lane
+//               sweep's, and the entries; with the tile sweeps (a handle's own batch) a level costs about a third
+// Measured, us an iteration, persistent / launches: 5-point 20^2 1 instance 56 / 144, 1,024 217 / 314; 7-point 8^3 64 instances
+// 59 / 138; 50^2 64 318 / 364; curl-curl 8^3 64 344 / 388, 10^3 64 787 / 599, 14^3 64 1,880 / 860; random sparse of 5,000 rows
+// 16 374 / 160; complex curl-curl 10^3 256 1,157 / 1,980, 14^3 16 2,260 / 1,200.
+struct BatchShape {
+    double instances, rows, nnz;   // of the whole batch
+    double max_rows, max_nnz;      // of its largest instance
+    double levels;                 // of the instance with most
+    int sms;
+    bool complex_values, tiles;    // tiles: the launches run the tile sweeps
+};
+inline double batch_persistent_us(const BatchShape &b) {
+    const bool c = b.complex_values;
+    const double lev = (c ? 1.2 : 1.3) * b.levels, row = c ? 0.080 : 0.042, ent = c ? 0.0062 : 0.0030;
+    const double alone = lev + row * b.max_rows + ent * b.max_nnz;
+    const double mean = lev + (row * b.rows + ent * b.nnz) / b.instances;
+    const double share = b.instances / ((c ? 0.92 : 0.30) * b.sms);
+    return share <= 1.0 ? alone : std::max(alone, mean * std::pow(share, c ? 0.68 : 0.34));
+}
+inline double batch_launches_us(const BatchShape &b) {
+    const bool c = b.complex_values;
+    // a quarter off: the persistent estimate is up to half too low where levels hold one row
+    if (b.tiles) return 0.75 * (c ? 90.0 + 1.5 * b.levels : 75.0 + 0.75 * b.levels);
+    const double width = b.rows / std::max(b.levels, 1.0);
+    const double level = std::min(c ? 3.6 + 1.0e-3 * width : 2.3 + 2.26e-4 * width, c ? 23.5 : 29.0);
+    return (c ? 114.0 : 90.0) + b.levels * level + (c ? 3.65e-5 : 7.2e-6) * b.nnz;
+}
+inline bool batch_persists(const BatchShape &b) { return batch_persistent_us(b) < batch_launches_us(b); }
 
 }  // namespace ssg
