@@ -393,7 +393,7 @@ bool Handle::push_ok(size_t elem) {
 bool Handle::tile_ok(Tri &a, Tri &b, size_t elem) {
     if (!use_inv_diag || sweep_mode != 0 || !push_auto || a.n == 0) return false;
     const int lanes = vtype == SSG_COMPLEX ? cl_group : 0;
-    if (lanes > 8) return false;
+    if (lanes != 0 && lanes != 4 && lanes != 8) return false;
     if (!narrow(a) || !narrow(b)) return false;
     return tile_plan(a, elem, lanes, stream) && tile_plan(b, elem, lanes, stream);
 }
@@ -730,7 +730,7 @@ Handle::TuneChoice Handle::autotune(bool keep_group, bool with_push) {
     // the push sweep sums each row in dependency-level order, not by lanes: a candidate
     // only when the summation order is free to change
     if (!keep_group && with_push) {
-        cand.push_back({4, 1, 0, 0.0});
+        cand.push_back({4, g0, 0, 0.0});  // its sums have no lanes: the handle's setting stays for what it does not serve
         cand.push_back({0, 4, 0, 0.0});  // the automatic choice: the tile sweep
     }
     const TuneChoice before{sweep_mode, swcfg.group, swcfg.cta_per_sm, 0.0};

@@ -429,6 +429,7 @@ TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, con
         return P;
     };
     if (n <= 0) return fail("no rows");
+    if (lanes != 0 && lanes != 4 && lanes != 8) return fail("not a number of lanes a row the records hold");
     if (T <= 0) T = tile_count(n, lanes);
     T = std::min(T, n);
     P.T = T;

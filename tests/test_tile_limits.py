@@ -86,3 +86,8 @@ def test_orders_that_scatter_dependencies_are_refused(lib, oracle, monkeypatch, 
         assert (got[0] == "") == served, got[0]
         if not served:
             assert "too many" in got[0]
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 16])
+def test_lanes_the_records_cannot_hold_are_refused(lib, oracle, lanes):
+    assert "lanes" in ask(lib, oracle, matrix("chain"), True, 16, lanes)
