@@ -264,10 +264,14 @@ int ssg_set_tuning(ssg_handle h, int key, int value);
 /* Autotuner (build addition): times the IC preconditioner of the current matrix
  * and factor for each candidate sweep schedule (sync-free with 4/8/16 lanes a row
  * and 2/4/8/16/automatic CTAs per SM; one-cluster level-synchronous and
- * neighbour-synchronised with 4/8 lanes), keeps the fastest in the handle's
- * tuning and reports it. keep_group = 1 keeps the current lanes per row, so
- * results stay bit-identical to an untuned run; otherwise they may change at
- * rounding level (a row's entries are summed in another order). */
+ * neighbour-synchronised with 4/8 lanes; one-cluster push; the automatic mode, for
+ * complex values with 4 and 8 lanes), keeps the fastest in the handle's tuning and
+ * reports it. keep_group = 1 keeps the way rows are summed, so results of either
+ * preconditioner stay bit-identical to an untuned run: where rows are summed by age
+ * (the automatic mode on real values, the push sweep) the mode stays, where they are
+ * summed by lanes the candidates are the schedules with the lanes now in use.
+ * Otherwise results may change at rounding level (a row's entries are summed in
+ * another order). */
 int ssg_autotune(ssg_handle h, int keep_group, int *mode, int *group, int *cta_per_sm, double *ms);
 
 /* ---- hot-path pieces on their own (host buffers) ---- */

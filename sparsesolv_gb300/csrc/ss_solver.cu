@@ -703,12 +703,15 @@ int Handle::solve(int method, double conv_cri, int max_ite, double normB, const 
 // Candidates differ only in schedule (which threads do which rows, and how they
 // wait): the sweep mode, the CTAs per SM of the sync-free sweep and, unless
 // keep_group, the lanes per row (a different lane count sums a row's entries in
-// a different order, so results change at rounding level). Each candidate is
-// run once to build its plans, then timed over three applications (median).
+// a different order, so results change at rounding level). With keep_group only
+// schedules that sum rows as the handle's present one does: by age (the automatic
+// mode on real values, mode 4) it stands alone, by lanes those of the same lanes.
+// Each candidate is run once to build its plans, then timed over three
+// applications (median).
 template <typename T>
 Handle::TuneChoice Handle::autotune(bool keep_group, bool with_push) {
     if (vtype < 0) throw Error{SSG_ERR_STATE, "no matrix set"};
-    if (n == 0) return TuneChoice{sweep_mode, swcfg.group, swcfg.cta_per_sm, 0.0};
+    if (n == 0) return TuneChoice{sweep_mode, swcfg.group, swcfg.cta_per_sm, 0.0, false};
     ensure_factor<T>(opt.accel_factor, opt.is_diag_scale != 0);
     ensure_work(sizeof(T));
     T *r = vec[1].as<T>(), *z = vec[3].as<T>();
@@ -717,44 +720,63 @@ Handle::TuneChoice Handle::autotune(bool keep_group, bool with_push) {
         SSG_CUDA(cudaMemcpyAsync(r, ones.data(), sizeof(T) * (size_t)n, cudaMemcpyHostToDevice, stream));
         SSG_CUDA(cudaStreamSynchronize(stream));
     }
-    const int g0 = cl_group;
+    constexpr bool cx = Sc<T>::is_complex;
+    const int own = swcfg.group ? swcfg.group : sweep_group(Lf);  // the sync-free sweep's lanes
     std::vector<TuneChoice> cand;
-    const std::vector<int> groups = keep_group ? std::vector<int>{g0} : std::vector<int>{4, 8, 16};
-    for (int g : groups)
-        for (int cps : {0, 2, 4, 8, 16}) cand.push_back({1, g, cps, 0.0});
-    for (int g : groups)
+    auto by_lanes = [&](int g) {
+        for (int cps : {0, 2, 4, 8, 16}) cand.push_back({1, g, cps, 0.0, false});
         if (g == 4 || g == 8) {
-            cand.push_back({2, g, 0, 0.0});
-            cand.push_back({3, g, 0, 0.0});
+            cand.push_back({2, g, 0, 0.0, false});
+            cand.push_back({3, g, 0, 0.0, false});
         }
-    // the push sweep sums each row in dependency-level order, not by lanes: a candidate
-    // only when the summation order is free to change
-    if (!keep_group && with_push) {
-        cand.push_back({4, g0, 0, 0.0});  // its sums have no lanes: the handle's setting stays for what it does not serve
-        cand.push_back({0, 4, 0, 0.0});  // the automatic choice: the tile sweep
+    };
+    if (!keep_group) {
+        for (int g : {4, 8, 16}) by_lanes(g);
+        if (with_push) {
+            cand.push_back({4, cl_group, 0, 0.0, true});
+            cand.push_back({0, 4, 0, 0.0, false});  // the automatic choice: the tile sweep
+            if (cx) cand.push_back({0, 8, 0, 0.0, false});
+        }
+    } else if (sweep_mode == 0 && !cx) {
+        const bool tiles = tile_ok(Lf, Ltb, sizeof(T));  // nothing of the sync-free sweep's to tune
+        cand.push_back({0, free_cfg(Lf).group ? free_cfg(Lf).group : own, swcfg.cta_per_sm, 0.0, true});
+        if (!tiles)
+            for (int cps : {0, 2, 4, 8, 16}) cand.push_back({0, cand[0].group, cps, 0.0, true});
+    } else if (sweep_mode == 4 && push_ok(sizeof(T))) {
+        cand.push_back({4, cl_group, swcfg.cta_per_sm, 0.0, true});
+    } else {
+        const bool cluster = sweep_mode >= 2 && cluster_ok(Lf, sizeof(T), true) && cluster_ok(Ltb, sizeof(T), true);
+        const bool wide = sweep_mode == 0 && !narrow(Lf);
+        const int g = cluster || (sweep_mode == 0 && !wide) ? cl_group : own;
+        by_lanes(g);
+        if (cx) cand.push_back({0, g, swcfg.cta_per_sm, 0.0, sweep_mode == 0});
     }
-    const TuneChoice before{sweep_mode, swcfg.group, swcfg.cta_per_sm, 0.0};
+    const TuneChoice before{sweep_mode, swcfg.group, swcfg.cta_per_sm, 0.0, false};
     const int cl_before = cl_group;
     const bool prof_on = prof.on;
     prof.on = false;
     // a batch's sweeps skip ended instances: time every row
     const int *row_inst = swcfg.row_inst;
     swcfg.row_inst = nullptr;
-    TuneChoice best{-1, 0, 0, 1e300};
-    auto restore = [&](const TuneChoice &k, int clg) {
+    TuneChoice best{-1, 0, 0, 1e300, false};
+    auto apply = [&](const TuneChoice &k) {
+        sweep_mode = k.mode;
+        swcfg.group = k.as_set ? before.group : k.group;
+        cl_group = k.as_set ? cl_before : k.group;
+        swcfg.cta_per_sm = k.cta_per_sm;
+    };
+    auto restore = [&](const TuneChoice &k) {
         prof.on = prof_on;
         swcfg.row_inst = row_inst;
-        sweep_mode = k.mode;
-        swcfg.group = k.group;
-        swcfg.cta_per_sm = k.cta_per_sm;
-        cl_group = clg;
+        apply(k);
+    };
+    auto undo = [&] {
+        restore(before);
+        cl_group = cl_before;
     };
     try {
         for (TuneChoice &c : cand) {
-            sweep_mode = c.mode;
-            swcfg.group = c.group;
-            cl_group = c.group;
-            swcfg.cta_per_sm = c.cta_per_sm;
+            apply(c);
             // a cluster candidate whose plan does not fit would time the sync-free sweep again
             if (c.mode == 4 && !push_ok(sizeof(T))) continue;
             if ((c.mode == 2 || c.mode == 3) && !(cluster_ok(Lf, sizeof(T), true) && cluster_ok(Ltb, sizeof(T), true)))
@@ -776,14 +798,14 @@ Handle::TuneChoice Handle::autotune(bool keep_group, bool with_push) {
             if (c.ms < best.ms) best = c;
         }
     } catch (...) {
-        restore(before, cl_before);
+        undo();
         throw;
     }
     if (best.mode < 0) {
-        restore(before, cl_before);
+        undo();
         throw Error{SSG_ERR_STATE, "autotune: no candidate ran"};
     }
-    restore(best, best.group);
+    restore(best);
     return best;
 }
 

@@ -175,6 +175,7 @@ struct Handle {
     struct TuneChoice {
         int mode, group, cta_per_sm;
         double ms;
+        bool as_set;  // the handle's lanes settings stay as they are
     };
     template <typename T>
     TuneChoice autotune(bool keep_group, bool with_push = true);
