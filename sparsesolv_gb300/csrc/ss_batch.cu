@@ -1535,13 +1535,13 @@ int solve_batched(Handle &h, Batch *&mb, uint64_t &mver, uint64_t &mpat, int pre
     }
     if (!mb) mb = new Batch(h.device);
     mb->h.prof.on = h.prof.on;  // profiling and the sweep schedule follow the owning handle
-    // lanes a row: one right-hand side runs the one-system schedule (the cluster sweep is
-    // fastest with 4 lanes for real rows; complex rows carry four times the multiply-adds
-    // and keep 8); several make the levels wide, and rows of more than 6 off-diagonal
-    // entries then run faster on 16 lanes
+    // lanes a row, where rows are summed by lanes (complex values, and real ones the tile sweeps do not serve): one
+    // right-hand side as one system (complex rows carry four times the multiply-adds and keep 8); several make the levels
+    // wide, and rows of more than 6 off-diagonal entries then ran faster on 16 lanes in the one-cluster sweeps
     int g = h.batch_group;
     if (!g) g = nrhs == 1 ? (h.vtype == SSG_COMPLEX ? 8 : 4) : ((h.nnz - h.n) > 12ll * h.n ? 16 : 8);
     mb->h.swcfg.group = mb->h.cl_group = g;
+    mb->h.lanes_cluster = h.batch_group;
     mb->h.swcfg.cta_per_sm = h.swcfg.cta_per_sm;
     mb->h.sweep_mode = h.sweep_mode;
     // a handle's own batch (mixed precision, several right-hand sides) serves one matrix:

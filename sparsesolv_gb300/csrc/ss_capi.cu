@@ -379,7 +379,7 @@ int ssg_set_tuning(ssg_handle hd, int key, int value) {
                 break;
             case SSG_TUNE_SWEEP_GROUP:
                 if (value != 0 && value != 4 && value != 8 && value != 16 && value != 32) return SSG_ERR_ARG;
-                h.swcfg.group = value;
+                h.swcfg.group = h.lanes_sweep = value;
                 break;
             case SSG_TUNE_SWEEP_BACKOFF_NS:
                 if (value < 0 || value > 100000) return SSG_ERR_ARG;
@@ -402,7 +402,7 @@ int ssg_set_tuning(ssg_handle hd, int key, int value) {
                 break;
             case SSG_TUNE_CLUSTER_GROUP:
                 if (value != 4 && value != 8 && value != 16 && value != 32) return SSG_ERR_ARG;
-                h.cl_group = value;
+                h.cl_group = h.lanes_cluster = value;
                 break;
             case SSG_TUNE_SPMV_GROUP:
                 if (value != 0 && value != 2 && value != 4 && value != 8 && value != 16 && value != 32) return SSG_ERR_ARG;

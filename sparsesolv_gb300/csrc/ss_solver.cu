@@ -347,13 +347,15 @@ static double tri_bytes(const Tri &T, size_t v, int vecs) {
 static constexpr double kNarrowRowsPerLevel = 4096.0;
 static bool narrow(const Tri &t) { return (double)t.n <= kNarrowRowsPerLevel * (double)t.nlev; }
 
-// What serves where the tile sweeps do not: the sync-free sweep, in the lanes a row (and so with the bits) of the
-// one-cluster sweep it replaced there as the automatic choice. Measured at 8 lanes a row, us forward: 10^3 190 (lockstep
-// cluster 263, push 221), 20^3 438 (583, 497), 41^3 960 (1,405, 1,088), 80^3 2,094 (4,435, 2,226), complex 33^3 1,277
-// (1,497). The one-cluster and push sweeps run where SSG_TUNE_SWEEP_MODE asks for them.
+// What serves where the tile sweeps do not: the sync-free sweep. Complex rows and the standalone batches' take the lanes (and
+// so the bits) of the one-cluster sweep it replaced there as the automatic choice, real rows 8 unless a number was asked for.
+// Measured at 8 lanes a row, us forward: 10^3 190 (lockstep cluster 263, push 221), 20^3 438 (583, 497), 41^3 960 (1,405,
+// 1,088), 80^3 2,094 (4,435, 2,226), complex 33^3 1,277 (1,497). The one-cluster and push sweeps run where
+// SSG_TUNE_SWEEP_MODE asks for them.
 SweepCfg Handle::free_cfg(const Tri &t) const {
     SweepCfg c = swcfg;
-    if (sweep_mode == 0 && narrow(t)) c.group = vtype == SSG_COMPLEX || !push_auto ? cl_group : 8;
+    if (sweep_mode == 0 && narrow(t))
+        c.group = vtype == SSG_COMPLEX || !push_auto ? cl_group : lanes_cluster ? lanes_cluster : lanes_sweep ? lanes_sweep : 8;
     return c;
 }
 

@@ -121,6 +121,9 @@ struct Handle {
     int cl_ring_bytes = 16 * 1024; // distributed shared-memory ring per CTA
     int cl_ring_bytes_p2p = 24 * 1024;  // its ring in mode 3 (producers may run ahead)
     int cl_group = 4;              // lanes per row in the cluster sweep
+    // lanes a row asked for (0: not), for what the automatic mode's sync-free sweep serves: SSG_TUNE_CLUSTER_GROUP (a
+    // handle's own batch: SSG_TUNE_BATCH_GROUP), else SSG_TUNE_SWEEP_GROUP
+    int lanes_cluster = 0, lanes_sweep = 0;
     // ic: an IC sweep (the only kind the neighbour-synchronised plan serves)
     bool cluster_ok(Tri &t, size_t elem, bool ic);
     SweepCfg free_cfg(const Tri &t) const;  // the sync-free sweep's launch shape
