@@ -203,9 +203,9 @@ void sweep_push(Tri &tri, const T *val, int mode, const T *rhs, const T *lvec, u
                 const KState *st, int *err, cudaStream_t s);
 
 // ss_tile.cu: whole-GPU tile sweeps (all modes; lvec: 1/diagonal, or D for SW_BWD_IC, per level-ordered row)
-// plan once per pattern and value size; false when a record does not fit (then another sweep serves)
+// plans of a pair of triangles, once per pattern and value size; false when one is refused (then another sweep serves)
 // lanes: 0 for real values, 4 or 8 for complex ones (the cluster sweep's lanes a row, and its bits)
-bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s);
+bool tile_plan(Tri &a, Tri &b, size_t elem_bytes, int lanes, cudaStream_t s);
 // epoch as for sweep_push; ticket: one int, reset here
 template <typename T>
 void sweep_tile(Tri &tri, const T *val, int mode, const T *rhs, const T *aux, const T *lvec, unsigned long long epoch,

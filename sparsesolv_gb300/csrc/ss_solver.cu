@@ -397,7 +397,7 @@ bool Handle::tile_ok(Tri &a, Tri &b, size_t elem) {
     const int lanes = vtype == SSG_COMPLEX ? cl_group : 0;
     if (lanes != 0 && lanes != 4 && lanes != 8) return false;
     if (!narrow(a) || !narrow(b)) return false;
-    return tile_plan(a, elem, lanes, stream) && tile_plan(b, elem, lanes, stream);
+    return tile_plan(a, b, elem, lanes, stream);
 }
 
 // z = (L D L^T)^{-1} r using vec[10] as the forward result

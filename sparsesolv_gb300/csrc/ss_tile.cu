@@ -47,6 +47,8 @@
 // word is set; the CTA then drains its copies and only goes along to the cluster's
 // barriers, until its cluster leaves together.
 #include <algorithm>
+#include <new>
+#include <utility>
 
 #include "sparsesolv_gb300.h"
 #include "ss_internal.cuh"
@@ -616,44 +618,39 @@ static int tile_sms() {
     return sms;
 }
 
-// The plan: once per pattern and value size, on the host (ss_tile_plan.cpp)
-bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s) {
-    const int elem = (int)elem_bytes, slot = elem == 4 ? 0 : elem == 8 ? 1 : 2;
-    TilePlan &P = T.tile[slot];
-    if (P.n != T.n || P.nnz != T.nnz || P.nlev != T.nlev || P.lanes != lanes) {
-        P.ready = P.failed = false;
-        P.lanes = lanes;
-        P.n = T.n;
-        P.nnz = T.nnz;
-        P.nlev = T.nlev;
-    }
-    if (P.ready) return true;
-    if (P.failed || T.n == 0) return false;
+static TilePlan &tile_slot(Tri &T, int elem) { return T.tile[elem == 4 ? 0 : elem == 8 ? 1 : 2]; }
+
+// another sweep serves the triangle; the buffers go back
+static void tile_refuse(TilePlan &P) {
+    for (DBuf *d : {&P.tiles, &P.groups, &P.halo, &P.rel, &P.dval, &P.dlv, &P.rec}) d->release();
+    P.ready = false;
+    P.failed = true;
+}
+
+static TilePlanHost tile_plan_of(const Tri &T, int elem, int lanes, const TileLimits &lim, cudaStream_t s) {
     std::vector<int> prp(T.n + 1), pci(T.nnz), ipos(T.n), level(T.n);
     SSG_CUDA(cudaMemcpyAsync(prp.data(), T.prp.p, sizeof(int) * (T.n + 1), cudaMemcpyDeviceToHost, s));
     SSG_CUDA(cudaMemcpyAsync(pci.data(), T.pci.p, sizeof(int) * (size_t)T.nnz, cudaMemcpyDeviceToHost, s));
     SSG_CUDA(cudaMemcpyAsync(ipos.data(), T.ipos.p, sizeof(int) * T.n, cudaMemcpyDeviceToHost, s));
     SSG_CUDA(cudaMemcpyAsync(level.data(), T.level.p, sizeof(int) * T.n, cudaMemcpyDeviceToHost, s));
     SSG_CUDA(cudaStreamSynchronize(s));
-    const TileLimits lim = tile_limits(lanes);
-    const TilePlanHost H =
-        tile_plan_host(T.n, T.nlev, prp.data(), pci.data(), ipos.data(), level.data(), T.lower, elem, lanes, 0,
-                       tile_cluster(tile_count(T.n, lanes), lanes), nullptr, &lim);
-    if (!H.ok) {
-        P.failed = true;
+    return tile_plan_host(T.n, T.nlev, prp.data(), pci.data(), ipos.data(), level.data(), T.lower, elem, lanes, 0,
+                          tile_cluster(tile_count(T.n, lanes), lanes), nullptr, &lim);
+}
+
+// false: no memory for it on the device
+static bool tile_upload(TilePlan &P, const TilePlanHost &H, cudaStream_t s) {
+    const std::pair<DBuf *, const std::vector<int> *> arr[] = {{&P.tiles, &H.tiles}, {&P.groups, &H.groups}, {&P.halo, &H.halo},
+                                                               {&P.rel, &H.rel},     {&P.dval, &H.dval},     {&P.dlv, &H.dlv}};
+    try {
+        for (auto &a : arr) a.first->ensure(sizeof(int) * (a.second->size() + 4));
+        P.rec.ensure((size_t)H.rec_bytes + 16);
+    } catch (const Error &) {
         return false;
     }
-    auto put = [&](DBuf &d, const std::vector<int> &h) {
-        d.ensure(sizeof(int) * (h.size() + 4));
-        if (!h.empty()) SSG_CUDA(cudaMemcpyAsync(d.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, s));
-    };
-    put(P.tiles, H.tiles);
-    put(P.groups, H.groups);
-    put(P.halo, H.halo);
-    put(P.rel, H.rel);
-    put(P.dval, H.dval);
-    put(P.dlv, H.dlv);
-    P.rec.ensure((size_t)H.rec_bytes + 16);
+    for (auto &a : arr)
+        if (!a.second->empty())
+            SSG_CUDA(cudaMemcpyAsync(a.first->p, a.second->data(), sizeof(int) * a.second->size(), cudaMemcpyHostToDevice, s));
     for (int t = 0; t < H.T; ++t)
         if (!H.rec[t].empty())
             SSG_CUDA(cudaMemcpyAsync(P.rec.as<unsigned char>() + H.rec_off[t], H.rec[t].data(), H.rec[t].size(),
@@ -664,14 +661,66 @@ bool tile_plan(Tri &T, size_t elem_bytes, int lanes, cudaStream_t s) {
     P.CS = H.CS;
     P.key_val = P.key_lv = nullptr;
     P.key_epoch = ~0ull;
-    P.ready = true;
+    return true;
+}
+
+// The plans of a pair of triangles: once per pattern and value size, on the host (ss_tile_plan.cpp). A plan that does not
+// fit, passes a limit or finds no memory, on the host or the device, is refused for good: the sync-free sweep, which needs
+// none of it, then serves the pair.
+bool tile_plan(Tri &a, Tri &b, size_t elem_bytes, int lanes, cudaStream_t s) {
+    const int elem = (int)elem_bytes;
+    bool all = true;
+    for (Tri *T : {&a, &b}) {
+        TilePlan &P = tile_slot(*T, elem);
+        if (P.n != T->n || P.nnz != T->nnz || P.nlev != T->nlev || P.lanes != lanes) {
+            P.ready = P.failed = false;
+            P.lanes = lanes;
+            P.n = T->n;
+            P.nnz = T->nnz;
+            P.nlev = T->nlev;
+        }
+        if (P.failed || T->n == 0) return false;
+        all = all && P.ready;
+    }
+    if (all) return true;
+    size_t here = 0, total = 0;
+    SSG_CUDA(cudaMemGetInfo(&here, &total));
+    const TileLimits lim = tile_limits(lanes, (long long)total);
+    Tri *tri[2] = {&a, &b};
+    TilePlanHost H[2];
+    for (int q = 0; q < 2; ++q) {
+        TilePlan &P = tile_slot(*tri[q], elem);
+        if (P.ready) continue;
+        try {
+            H[q] = tile_plan_of(*tri[q], elem, lanes, lim, s);
+        } catch (const std::bad_alloc &) {
+        }
+        if (!H[q].ok) {
+            tile_refuse(P);
+            return false;
+        }
+    }
+    for (int q = 0; q < 2; ++q) {
+        TilePlan &P = tile_slot(*tri[q], elem);
+        if (P.ready) continue;
+        if (!tile_upload(P, H[q], s)) {
+            tile_refuse(P);
+            // the other one is of no use without it
+            if (q == 1 && H[0].ok) {
+                tile_refuse(tile_slot(a, elem));
+                tile_slot(a, elem).failed = false;
+            }
+            return false;
+        }
+        P.ready = true;
+    }
     return true;
 }
 
 template <typename T>
 void sweep_tile(Tri &tri, const T *val, int mode, const T *rhs, const T *aux, const T *lvec, unsigned long long epoch,
                 T *out, T *out2, int *ticket, const KState *st, int *err, cudaStream_t s) {
-    TilePlan &P = tri.tile[sizeof(T) == 4 ? 0 : sizeof(T) == 8 ? 1 : 2];
+    TilePlan &P = tile_slot(tri, (int)sizeof(T));
     if (tri.n == 0) return;
     if (!P.ready || P.n != tri.n || P.nnz != tri.nnz || P.nlev != tri.nlev)
         throw Error{SSG_ERR_STATE, "tile sweep without a plan for this triangle"};

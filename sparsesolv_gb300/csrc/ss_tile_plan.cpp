@@ -70,7 +70,11 @@ int tile_cluster(int T, int lanes) { return lanes || T < 8 ? 1 : 8; }
 // orders shuffled within a window have few chunks and many of them. Far entries a row, us tiles / sync-free, complex 24^3 with
 // windows of 500, 2,000 and 6,000 rows: 0.04 1,459 / 1,712, 0.6 1,653 / 1,306, 3.7 1,574 / 734; real 40^3: 0.01 896 / 1,986,
 // 0.08 1,537 / 1,739, 0.07 1,713 / 1,328.
-TileLimits tile_limits(int lanes) { return {lanes ? 1.0 : 3.0, 0.1}; }
+// Memory. A record holds 32 lanes whatever its group has, so its bytes over the triangle's CSR bytes are about 2 where levels
+// are wide (breadth-first curl-curl 80^3 1.9, 27-point 80^3 1.6, complex 4 to 5), and up to 20 where a level is one row
+// (tridiagonal 17, bands 14 to 16); the tiles are 3 to 4 times faster there all the same (band of 16, 50,000 rows: 12 against
+// 46 ms). The records, which the host holds too while it plans, may take a sixteenth of the device's memory (17 GB).
+TileLimits tile_limits(int lanes, long long device_bytes) { return {lanes ? 1.0 : 3.0, 0.1, device_bytes / 16}; }
 
 namespace {
 
@@ -450,7 +454,7 @@ TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, con
     // a limit passed: the passes run out without work. Each limit is on a maximum or a sum, so the outcome does not depend on
     // the threads.
     std::atomic<const char *> over{nullptr};
-    std::atomic<long long> nfar{0};
+    std::atomic<long long> nfar{0}, bytes{0};
     const double max_chunks = lim ? lim->chunks_per_level * std::max(nlev, 1) : 0.0;
     const double max_far = lim ? lim->far_per_row * n : 0.0;
     auto work = [&](int q) {
@@ -469,6 +473,7 @@ TilePlanHost tile_plan_host(int n, int nlev, const int *prp, const int *pci, con
                     } else if (!halo[t].why) {
                         plan_tile(C, first(t), first(t + 1), halo[t], push[t / CS], *S, out[t]);
                         if (lim && (double)(nfar += out[t].nfar) > max_far) over = "too many far entries";
+                        if (lim && (bytes += (long long)out[t].rec.size()) > lim->bytes) over = "records too large";
                     }
                 } catch (...) {
                     errs[q] = std::current_exception();

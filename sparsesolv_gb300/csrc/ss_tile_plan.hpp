@@ -131,8 +131,9 @@ int tile_cluster(int T, int lanes);
 struct TileLimits {
     double chunks_per_level;  // halo chunks of the tile with most of them, over the triangle's levels
     double far_per_row;       // far entries, over the rows
+    long long bytes;          // of the records
 };
-TileLimits tile_limits(int lanes);
+TileLimits tile_limits(int lanes, long long device_bytes);
 // n rows: prp/pci the level-ordered rows (columns as row ids, the diagonal included), ipos[row] position of a row,
 // level[row]; lower: solve order is ascending rows. lanes: 0 sums by age, 4 or 8 by lanes. T tiles (<= 0: tile_count), CS
 // of them a cluster. lim: null for a plan at any cost.

@@ -50,7 +50,10 @@ def matrix(name):
     return A
 
 
-def ask(lib, oracle, A, lower, elem, lanes):
+DEVICE = 284 << 30
+
+
+def ask(lib, oracle, A, lower, elem, lanes, device_bytes=DEVICE, size=None):
     rp, ci = A.indptr.astype(np.int32), A.indices.astype(np.int32)
     n = len(rp) - 1
     trp, tci, _ = oracle.triangle(rp, ci, lower)
@@ -63,7 +66,8 @@ def ask(lib, oracle, A, lower, elem, lanes):
     np.cumsum(lens, out=prp[1:])
     pci = np.ascontiguousarray(tci[np.repeat(trp[:-1][perm] - prp[:-1], lens) + np.arange(prp[-1])], np.int32)
     ptr = [a.ctypes.data_as(ctypes.c_void_p) for a in (prp, pci, ipos, level)]
-    return lib.tile_limits_check(n, len(lptr) - 1, *ptr, int(lower), elem, lanes).decode()
+    return lib.tile_limits_check(n, len(lptr) - 1, *ptr, int(lower), elem, lanes, ctypes.c_longlong(device_bytes),
+                                 size if size is None else ctypes.byref(size)).decode()
 
 
 # (matrix, lanes a row: 0 real, 4 complex, 8 complex; served by the tile sweep)
@@ -91,3 +95,17 @@ def test_orders_that_scatter_dependencies_are_refused(lib, oracle, monkeypatch, 
 @pytest.mark.parametrize("lanes", [1, 2, 16])
 def test_lanes_the_records_cannot_hold_are_refused(lib, oracle, lanes):
     assert "lanes" in ask(lib, oracle, matrix("chain"), True, 16, lanes)
+
+
+@pytest.mark.parametrize("name,lanes", [("voxel12", 0), ("voxel12", 4), ("chain", 0)])
+def test_records_beyond_their_share_of_the_device_are_refused(lib, oracle, monkeypatch, name, lanes):
+    """The records may take a sixteenth of the device's memory: at that line the plan is made, a byte below it is not."""
+    A = matrix(name)
+    size = ctypes.c_longlong(0)
+    assert ask(lib, oracle, A, True, 16 if lanes else 8, lanes, size=size) == ""
+    for threads in ("1", "8"):
+        monkeypatch.setenv("SSG_PLAN_THREADS", threads)
+        assert ask(lib, oracle, A, True, 16 if lanes else 8, lanes, 16 * size.value) == ""
+        assert ask(lib, oracle, A, True, 16 if lanes else 8, lanes, 16 * size.value - 1) == "records too large"
+    csr = (8 + 4 + 8 * (lanes > 0)) * sp.tril(A).nnz
+    assert size.value <= 20 * csr  # the inflation the limit is stated with
