@@ -13,7 +13,7 @@ namespace ssg {
 // Measured, us a forward and a backward sweep together, k_sweep / k_sweep_wide, by rows a level:
 //   FP64 batches, 8 lanes   5-point 100^2 16,000 1,213 / 1,744, 21,000 1,568 / 1,734, 30,000 2,170 / 1,753; 7-point 24^3 20,900
 //                           584 / 670, 30,000 802 / 693; 27-point 14^3 16,000 612 / 965; 1,024 curl-curl systems of 8 to 32
-//                           voxels 58,000: a whole pass 1,033 / 683 ms
+//                           voxels 58,000: a whole pass 1,033 / 633 ms
 //   FP64, one system        random order, 7-point 10,300 102 / 106, 14,600 126 / 112, 18,100 154 / 119, 22,000 189 / 139; 5-point
 //                           11,400 89 / 81; curl-curl (16 lanes) 7,300 422 / 481, 11,200 594 / 554
 //   complex batches, 8      5-point 100^2 9,000 2,972 / 3,310, 12,000 3,700 / 3,416, 16,000 4,664 / 3,561; 27-point 14^3 9,000

@@ -123,7 +123,6 @@ __device__ __forceinline__ void tl_give(cplxf *p, cplxf v) {
     st_vol(&p->y, unsent(v.y));
 }
 
-// a warp that tests a staged group's barrier has itself taken the group staged there before, so the parity is unambiguous
 // CTAs of a cluster: a value stored into another one's shared memory, and barriers of all
 __device__ __forceinline__ unsigned tl_rank() {
     unsigned r;
@@ -279,7 +278,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_sweep_tile(TileArgs a) {
                     return;
                 }
         };
-        // group g's record, once staged; null: give up
+        // group g's record, once staged; null: give up. A warp that tests a staged group's barrier has itself taken the group
+        // staged there before, so the parity is unambiguous.
         auto record = [&](int g) -> const unsigned char * {
             const unsigned bar = full + 8u * (g % TS_NM);
             const unsigned par = (unsigned)((g / TS_NM) & 1);

@@ -110,7 +110,8 @@ SSG_HD inline int ts_col(int q, int lane, int blk, int elem) {
 
 // tiles: per tile {first group, groups, first halo chunk, halo chunks}
 // groups: per group {record offset / 16, record bytes / 16, ring offset / 16, group that must be done before the copy}
-// halo: row ids, 32 a chunk (-1: padding, -2: stored into its slot by a tile of the cluster); rel: per 32 of them the group up to which all must be done before they are delivered (-1: none)
+// halo: row ids, 32 a chunk (-1: padding, -2: stored into its slot by a tile of the cluster); rel: per 32 of them the group up
+// to which all must be done before they are delivered (-1: none)
 // dval: per entry of the level-ordered triangle its element index in rec, -1: the diagonal;
 // dlv: per level-ordered row the element index of its lv
 struct TilePlanHost {
