@@ -26,7 +26,7 @@
 //     the halo ring, or polls the ring for a value the cluster stores there; the
 //     count of values here, in list order, is published;
 //   * one warp stages the groups' records with bulk copies as ring space frees.
-// Waits inside a CTA are one load of the progress words and one vote.
+// Waits inside a CTA are one load of the progress words, one vote and a warp barrier.
 // Values go between CTAs one aligned 4- or 8-byte store at a time, which is
 // single-copy atomic, so a value is its own flag and no fence is needed.
 //
@@ -38,7 +38,7 @@
 //   curl-curl, real:  10^3  54 / 55 [221 / 222], 20^3 120 / 123 [496 / 501],
 //                     41^3 322 / 325 [1,095 / 1,090], 80^3 908 / 904 [2,237 / 2,195] (push); without clusters 123 / 127,
 //                     375 / 379 and 1,101 / 994
-//   SGS pair, 48^3:   490 / 483 [1,834 / 1,810] (lockstep)
+//   SGS pair, 48^3:   439 / 417 [1,834 / 1,810] (lockstep)
 //   eddy currents:    33^3 640 / 813 [1,638 / 1,525], 60^3 1,310 / 1,668 [3,616 / 3,338] (lockstep); 707 / 903 and
 //                     1,490 / 1,830 with a lane holding both parts of a sum and 2.5 times fewer tiles
 //   FP32, 44^3:       206 / 210 [504 / 498] (push)
